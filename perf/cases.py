@@ -393,7 +393,7 @@ class _Exact:
         return -self.kappa * out
 
     def R(self, psi, sign=1, inverse=False):
-        f = torch.tensor([1, 1, -1, -1], device="cuda").reshape(4, 1, 1) * (1j * self.mubar * sign)
+        f = torch.tensor([1, 1, -1, -1], dtype=torch.float64, device="cuda").reshape(4, 1, 1) * (1j * self.mubar * sign)
         return (1 - f) * psi / (1 + self.mubar ** 2) if inverse else (1 + f) * psi
 
     @staticmethod
