@@ -94,6 +94,7 @@ struct c2q_gauge {
     c2q_ctx* ctx = nullptr;
     c2q_lattice lat{};
     c2q::Geom geom{};
+    c2q::HopCoef coef{};  // hop phases of the lattice (scale unset)
     // [0] FP64 18-real, [1] FP64 12-real, [2] FP32 18-real, [3] FP32 12-real, [4] FP16 12-real,
     // [5] FP16 18-real; [6..9] the FP32 / FP16 kinds of the field in the temporal gauge
     c2q::GaugeStore store[10];
@@ -146,6 +147,9 @@ bool same_lattice(const c2q_lattice& a, const c2q_lattice& b);
 double as_build_option(double v);
 // Hop coefficients for one launch: -kappa * boundary phase (and chemical potential on T).
 HopCoef hop_coef(const c2q_lattice& lat, double kappa);
+// the same for the gauge field's lattice, from the phases it keeps (forming them
+// goes through the text of sixteen numbers, some microseconds of each launch)
+HopCoef hop_coef(const c2q_gauge* g, double kappa);
 EpiArgs diag_epi(double mubar, int which, int gamma5);
 
 // gauge storage for operator sweeps at precision `prec` (FP16 links are always 12-real)
@@ -153,7 +157,9 @@ int gkind_for(int prec, int rec12);
 
 // ---- fields ----
 // Allocate a spinor field of storage precision `prec` (stream-ordered allocation).
-int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f);
+// Its contents are undefined unless `clear`: work fields are written whole before
+// they are read, and no kernel reads the padding after the last site.
+int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f, bool clear = false);
 void field_free(c2q_spinor_eo* f);
 size_t field_bytes(const Geom& g, int prec);
 int gauge_ensure(c2q_gauge* g, int kind);  // builds a lower-precision copy on first use

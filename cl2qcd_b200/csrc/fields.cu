@@ -93,6 +93,13 @@ HopCoef hop_coef(const c2q_lattice& lat, double kappa)
     return c;
 }
 
+HopCoef hop_coef(const c2q_gauge* g, double kappa)
+{
+    HopCoef c = g->coef;
+    c.scale   = -kappa;
+    return c;
+}
+
 // Site-diagonal factors (ocl_kernel/fermionmatrix_eo_m.cl:22-109, _m_merged.cl:22-64):
 // spins 0,1 get f1, spins 2,3 get f2, the inverse carries 1/(1+mubar^2).
 EpiArgs diag_epi(double mubar, int which, int gamma5)
@@ -119,7 +126,7 @@ size_t field_bytes(const Geom& g, int prec)
     return lanes * 3 * 16 + lanes * 4;  // FP16 lanes + float norms
 }
 
-int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f)
+int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f, bool clear)
 {
     f->ctx  = ctx;
     f->lat  = lat;
@@ -130,8 +137,7 @@ int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f
     const size_t bytes = field_bytes(f->geom, prec);
     void* p            = nullptr;
     C2Q_CUDA(ctx, cudaMallocAsync(&p, bytes, ctx->stream));
-    // zero the padding once so that reductions over whole lanes never see garbage
-    C2Q_CUDA(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));
+    if (clear) C2Q_CUDA(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));
     f->data = p;
     f->norm = prec == 16 ? reinterpret_cast<float*>(static_cast<char*>(p) + (size_t)f->geom.stride * 3 * 16) : nullptr;
     f->owned = true;
@@ -470,7 +476,7 @@ static int dslash_typed(c2q_ctx* ctx, const c2q_gauge* g, int gkind, c2q_spinor_
     prm.y          = sptr<P>(dot.y);
     prm.gauge      = g->store[gkind].data;
     prm.g          = out->geom;
-    prm.c          = hop_coef(out->lat, kappa);
+    prm.c          = hop_coef(g, kappa);
     prm.e          = e;
     prm.out_parity = out_parity;
     const int blocks = (out->geom.seo + 127) / 128;
@@ -875,6 +881,7 @@ C2Q_EXPORT int c2q_gauge_create(c2q_ctx* ctx, const c2q_lattice* lat, c2q_gauge*
         delete g;
         return fail(ctx, C2Q_BAD_ARG, "lattice extents must be even and >= 2");
     }
+    g->coef            = hop_coef(*lat, 0.0);
     const size_t bytes = (size_t)8 * 9 * g->geom.stride * 16;
     cudaError_t e      = cudaMalloc(&g->store[G64].data, bytes);
     if (e != cudaSuccess) {
@@ -961,7 +968,7 @@ C2Q_EXPORT int c2q_spinor_eo_create_precision(c2q_ctx* ctx, const c2q_lattice* l
     if (precision != 64 && precision != 32 && precision != 16)
         return fail(ctx, C2Q_BAD_ARG, "precision must be 64, 32 or 16");
     c2q_spinor_eo* f = new c2q_spinor_eo();
-    int rc           = field_alloc(ctx, *lat, precision, f);
+    int rc           = field_alloc(ctx, *lat, precision, f, true);
     if (rc) {
         delete f;
         return rc;
