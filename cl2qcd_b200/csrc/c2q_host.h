@@ -271,6 +271,57 @@ int apply_operator_batch(c2q_ctx* ctx, int op, int n, c2q_spinor_eo* const* out,
                          c2q_spinor_eo* const* tmp1, c2q_spinor_eo* const* tmp2, int dot_mode,
                          const c2q_spinor_eo* const* y, int fin, SolverScalars* const* sc, int* sweeps,
                          c2q_spinor_eo* const* r_update = nullptr, c2q_spinor_eo* const* x_update = nullptr);
+// Iterations of the mixed-precision CG on QplusQminus_eo in one cooperative
+// launch (pcg.cuh), for the right-hand sides of a batch that share a field in
+// the temporal gauge: from their search directions p, FP32 residuals rs and
+// solution increments xs and device scalars sc, until one of them needs the
+// host (a reliable update is due, or its residual is no number) or `iters` are
+// done.  Bitwise the iterates of apply_operator_batch with mix_p.
+struct PcgBatch {
+    int n = 0;
+    c2q_spinor_eo *p[MAX_BATCH] = {}, *t1[MAX_BATCH] = {}, *t2[MAX_BATCH] = {}, *rs[MAX_BATCH] = {},
+                  *xs[MAX_BATCH] = {};
+    SolverScalars* sc[MAX_BATCH] = {};
+    double thr[MAX_BATCH] = {}, maxrr[MAX_BATCH] = {};
+    bool skip[MAX_BATCH] = {};  // the residual before the first iteration is not to be judged
+    double kappa = 0, mubar = 0, delta = 0;
+    int action = 0, first = 0, iters = 0;
+    void* ctl = nullptr;  // pcg_ctl_bytes() of device memory
+};
+struct PcgResult {
+    int iters;  // done; the last one judged the residual of the one before
+    double judged[MAX_BATCH], maxrr[MAX_BATCH];
+    int flag[MAX_BATCH];
+};
+// *most: the largest batch that takes these iterations on a lattice of geometry g
+// -- every tile of every right-hand side needs a resident block of its own (one
+// wave).  With more, a phase runs a second, partly empty wave between two
+// barriers and the ordinary launches are as fast or faster: FP16, per iteration
+// with its share of the reliable updates, 16^3x32 (256 tiles) 53 us against 69 us,
+// 20^3x40 (625 tiles) 110 against 104, four sources at 16^3x32 165 against 144.
+int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* most);
+size_t pcg_ctl_bytes();
+int pcg_run(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B, PcgResult* out);
+// Iterations of the FP64 CG on QplusQminus_eo in one cooperative launch
+// (pcg64.cu), with the context's solver scalars: until a judged residual is
+// below thr (from iteration min_iter on) or no number, or `iters` are done.
+struct Pcg64Solve {
+    c2q_spinor_eo *x, *r, *p, *t1, *t2;
+    double kappa, mubar;
+    int action;
+    int iter0, iters, min_iter;
+    int p_ready;      // p is up to date for the first iteration (a refresh set it)
+    int lag;          // 1: judge each residual one iteration later (skip: not at the first iteration)
+    int skip;
+    int check_every;  // lag 0: judge iterations whose number is a multiple of this, at once
+    double thr;
+};
+struct Pcg64Result {
+    int iters, stop;
+    double judged;
+};
+bool pcg64_applies(const c2q_ctx* ctx, int op, const c2q_gauge* g);
+int pcg64_run(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const Pcg64Solve& S, Pcg64Result* out);
 // an event for per-launch profiling (from the context's pool)
 cudaEvent_t profile_event(c2q_ctx* ctx);
 

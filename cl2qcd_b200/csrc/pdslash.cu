@@ -195,6 +195,28 @@ PkGeom pk_geom(const Geom& g)
     return p;
 }
 
+// what the slots' stencils of a launch on `ref`'s lattice and precision have in common
+void pk_stencil_args(const c2q_spinor_eo* ref, const c2q_gauge* g, int gkind, double kappa, PkStencil* st)
+{
+    st->gauge = g->store[gkind].data;
+    st->g     = pk_geom(ref->geom);
+    st->c     = hop_coef(g, kappa);
+    if (gkind_is_tg(gkind)) {
+        // temporal gauge: the T phases sit in the transformation, the last slice's
+        // T hop carries lambda
+        st->tg     = 1;
+        st->lam_re = g->tg_lam_re;
+        st->lam_im = g->tg_lam_im;
+        for (int d = 0; d < 2; ++d) {
+            st->c.re[0][d] = 1.0;
+            st->c.im[0][d] = 0.0;
+        }
+        st->c.real_mask = 0xFFu;
+    }
+    // FP16: links in units of 1/32767 and neighbour spinors in units of norm/32767
+    if (ref->prec == 16) st->c.scale *= 1.0 / (32767.0 * 32767.0);
+}
+
 static void fill_field(const c2q_spinor_eo* f, const void** d, const float** n)
 {
     *d = f ? f->data : nullptr;
@@ -219,23 +241,7 @@ static int pk_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PkBatch&
     }
     prm.nrhs       = B.n;
     prm.pdl        = ctx->pdl;
-    prm.gauge      = g->store[gkind].data;
-    prm.g          = pk_geom(ref->geom);
-    prm.c          = hop_coef(ref->lat, B.kappa);
-    if (gkind_is_tg(gkind)) {
-        // temporal gauge: the T phases sit in the transformation, the last slice's
-        // T hop carries lambda
-        prm.tg     = 1;
-        prm.lam_re = g->tg_lam_re;
-        prm.lam_im = g->tg_lam_im;
-        for (int d = 0; d < 2; ++d) {
-            prm.c.re[0][d] = 1.0;
-            prm.c.im[0][d] = 0.0;
-        }
-        prm.c.real_mask = 0xFFu;
-    }
-    // FP16: links in units of 1/32767 and neighbour spinors in units of norm/32767
-    if (P == 16) prm.c.scale *= 1.0 / (32767.0 * 32767.0);
+    pk_stencil_args(ref, g, gkind, B.kappa, &prm);
     prm.e          = B.e;
     prm.out_parity = B.out_parity;
     prm.ntiles = (prm.g.H + PK_THREADS - 1) / PK_THREADS;

@@ -55,18 +55,22 @@ struct PkGeom {
     FastDiv div_nsh, div_ns;
 };
 
-template <int P>
-struct PkParams {
-    PkRhs r[PK_MAX_RHS];
-    int nrhs;
+// What every slot's stencil of a launch has in common.
+struct PkStencil {
     const void* gauge;
     PkGeom g;
     HopCoef c;
+    int tg;                 // the gauge field is in the temporal gauge (PH_TG)
+    double lam_re, lam_im;  // PH_TG: weight of the T hop leaving the last time slice
+};
+
+template <int P>
+struct PkParams : PkStencil {
+    PkRhs r[PK_MAX_RHS];
+    int nrhs;
     EpiArgs e;
     int out_parity;
     int ntiles;  // tiles of PK_THREADS slots per right-hand side
-    int tg;                 // the gauge field is in the temporal gauge (PH_TG)
-    double lam_re, lam_im;  // PH_TG: weight of the T hop leaving the last time slice
     RedArgs red;
     int pdl;                // launched as a dependent launch (launch_dep)
 };
@@ -460,7 +464,7 @@ __device__ __forceinline__ Kc uniform_weight(double re, double im)
 
 // hop q = 2 mu + back, with the phase pattern resolved
 template <int P, int NL, int MU, bool BACK, bool SWP, int PH>
-__device__ __forceinline__ void pk_hop_ph(C2 acc[12], const PkParams<P>& prm, const uint4* st)
+__device__ __forceinline__ void pk_hop_ph(C2 acc[12], const PkStencil& prm, const uint4* st)
 {
     const int d  = BACK ? 1 : 0;
     const Kc w   = uniform_weight(prm.c.re[MU][d], prm.c.im[MU][d]);
@@ -481,7 +485,7 @@ __device__ __forceinline__ void pk_hop_ph(C2 acc[12], const PkParams<P>& prm, co
 // lattice; the other lane steps between two inner slices, where the stored
 // link is the identity and the weight 1.
 template <int P, int NL, bool BACK>
-__device__ __forceinline__ void pk_hop_tg_fold(C2 acc[12], const PkParams<P>& prm, const uint4* st)
+__device__ __forceinline__ void pk_hop_tg_fold(C2 acc[12], const PkStencil& prm, const uint4* st)
 {
     const float lr = (float)prm.lam_re, li = (float)prm.lam_im;
     const Kc w     = BACK ? Kc{make_float2(lr, 1.0f), make_float2(-li, 0.0f), make_float2(-lr, -1.0f),
@@ -498,11 +502,188 @@ __host__ __device__ constexpr int pk_link_bytes()
     return P == 16 ? (NL == 6 ? 48 : 72) : 16 * NL;
 }
 
+// The hopping sum of one slot of parity po into acc, streamed through the
+// thread's ring (a ring of S::STAGES stages at `mine`, the stage of hop q at
+// q % S::STAGES).  extra(q, st), q = 8 and 9, stages the epilogue operands into
+// the slots after the last hops; on return every staged copy has landed.
+template <int P, int NL, int PH, class S, class Extra>
+__device__ __forceinline__ void pk_stencil(C2 acc[12], const PkStencil& prm, const void* in, const float* in_norm,
+                                           int po, int j, uint4* mine, Extra&& extra)
+{
+    static_assert(S::STAGES == 2 || S::STAGES == 3, "the prologue below issues one or two stages");
+    const PkGeom& g = prm.g;
+    // coordinates of slot j (site 0 at time t < NT/2; site 1 at t + NT/2)
+    const unsigned r1 = fdiv((unsigned)j, g.div_nsh);
+    const int xh      = j - (int)r1 * g.nsh;
+    const unsigned r2 = fdiv(r1, g.div_ns);
+    const int y       = (int)r1 - (int)r2 * g.ns;
+    const int t       = (int)fdiv(r2, g.div_ns);
+    const int z       = (int)r2 - t * g.ns;
+    const int x       = 2 * xh + ((po + y + z + t) & 1);
+    const int yzt     = j - xh;
+    const int ss      = g.ss;
+
+    const size_t grp      = (size_t)pk_link_bytes<P, NL>() * ss;
+    const char* gb        = static_cast<const char*>(prm.gauge);
+    const char* fwd_links = gb + (size_t)(po * 4) * grp;
+    const char* bwd_links = gb + (size_t)((1 - po) * 4) * grp;
+
+    // neighbour slot and link slot of the 8 hops (q = 2 mu + back); across
+    // the fold in time the neighbour slot holds the pair swapped
+    const bool fold_f = t + 1 == g.nt2, fold_b = t == 0;
+    const int base    = j - g.vs_h * t;
+    int nb[8];
+    nb[0]        = fold_f ? base : j + g.vs_h;
+    nb[1]        = fold_b ? base + g.vs_h * (g.nt2 - 1) : j - g.vs_h;
+    const int xp = x + 1 == g.ns ? 0 : x + 1, xm = x == 0 ? g.ns - 1 : x - 1;
+    nb[2]        = (xp >> 1) + yzt;
+    nb[3]        = (xm >> 1) + yzt;
+    const int row = g.nsh, pl = g.nsh * g.ns;
+    nb[4]         = y + 1 == g.ns ? j - (g.ns - 1) * row : j + row;
+    nb[5]         = y == 0 ? j + (g.ns - 1) * row : j - row;
+    nb[6]         = z + 1 == g.ns ? j - (g.ns - 1) * pl : j + pl;
+    nb[7]         = z == 0 ? j + (g.ns - 1) * pl : j - pl;
+
+    // stage q: hops 0..7, then the epilogue operands (q = 8 and 9); every
+    // index below is a compile-time constant
+    auto issue = [&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        uint4* st       = mine + (size_t)((q % S::STAGES) * S::CH) * PK_THREADS;
+        if constexpr (q < 8) {
+            constexpr bool back = q & 1;
+            stage_spinor<P>(st, in, in_norm, ss, nb[q]);
+            // temporal gauge: the T links between inner slices are the identity
+            if (PH != PH_TG || q >= 2 || (back ? fold_b : fold_f))
+                stage_link<P, NL>(st, (back ? bwd_links : fwd_links) + (size_t)(q >> 1) * grp, ss, back ? nb[q] : j);
+        } else {
+            extra(qc, st);
+        }
+        cp_commit();
+    };
+
+#pragma unroll
+    for (int c = 0; c < 12; ++c) acc[c] = C2{bc2(0.f), bc2(0.f)};
+
+    auto step = [&](auto hc) {
+        constexpr int h = decltype(hc)::value;
+        if constexpr (h + S::STAGES - 1 <= 9)
+            issue(std::integral_constant<int, h + S::STAGES - 1>{});
+        else
+            cp_commit();
+        cp_wait<S::STAGES - 1>();
+        const uint4* st = mine + (size_t)((h % S::STAGES) * S::CH) * PK_THREADS;
+        constexpr int mu = h >> 1;
+        constexpr bool back = h & 1;
+        if constexpr (mu == 0 && PH == PH_TG) {
+            if (back ? fold_b : fold_f)
+                pk_hop_tg_fold<P, NL, back>(acc, prm, st);
+            else
+                pk_hop_id<P, back>(acc, st, 1.0f);
+        } else if constexpr (mu == 0) {
+            if (back ? fold_b : fold_f)
+                pk_hop_ph<P, NL, 0, back, true, PH>(acc, prm, st);
+            else
+                pk_hop_ph<P, NL, 0, back, false, PH>(acc, prm, st);
+        } else {
+            pk_hop_ph<P, NL, mu, back, false, PH>(acc, prm, st);
+        }
+    };
+    issue(std::integral_constant<int, 0>{});
+    if constexpr (S::STAGES > 2) issue(std::integral_constant<int, 1>{});
+    step(std::integral_constant<int, 0>{});
+    step(std::integral_constant<int, 1>{});
+    step(std::integral_constant<int, 2>{});
+    step(std::integral_constant<int, 3>{});
+    step(std::integral_constant<int, 4>{});
+    step(std::integral_constant<int, 5>{});
+    step(std::integral_constant<int, 6>{});
+    step(std::integral_constant<int, 7>{});
+    if constexpr (S::STAGES == 2) issue(std::integral_constant<int, 9>{});
+    cp_wait<0>();
+}
+
+// Epilogues on the hopping sum: h = sc * acc (sc = -kappa, times the FP16 scales).
+__device__ __forceinline__ void pk_epi_plain(C2 acc[12], float sc)
+{
+#pragma unroll
+    for (int c = 0; c < 12; ++c) acc[c] = C2{mul2(acc[c].re, bc2(sc)), mul2(acc[c].im, bc2(sc))};
+}
+__device__ __forceinline__ void pk_epi_diag(C2 acc[12], const EpiArgs& e, float sc)
+{
+#pragma unroll
+    for (int c = 0; c < 12; ++c) {
+        const float fr = (float)(c < 6 ? e.f1re : e.f2re) * sc;
+        const float fi = (float)(c < 6 ? e.f1im : e.f2im) * sc;
+        const C2 a     = acc[c];
+        acc[c]         = C2{fma2(a.re, bc2(fr), mul2(a.im, bc2(-fi))), fma2(a.im, bc2(fr), mul2(a.re, bc2(fi)))};
+    }
+}
+// [g5] (f x - sc acc), x staged at s8; FP16 x as exact integers q with the
+// per-site scale folded into f, the sign of g5 folded into the coefficients
+template <int P>
+__device__ __forceinline__ void pk_epi_axpy(C2 acc[12], const EpiArgs& e, float sc, const uint4* s8)
+{
+    C2 xv[12];
+    float2 xs;
+    staged_operand<P>(s8, xv, &xs);
+#pragma unroll
+    for (int c = 0; c < 12; ++c) {
+        const float gs  = (e.gamma5 && c >= 6) ? -1.0f : 1.0f;
+        const float2 fr = mul2(bc2(gs * (float)(c < 6 ? e.f1re : e.f2re)), xs);
+        const float2 fi = mul2(bc2(gs * (float)(c < 6 ? e.f1im : e.f2im)), xs);
+        const float2 nf = mul2(bc2(-gs * (float)(c < 6 ? e.f1im : e.f2im)), xs);
+        const float ms  = -gs * sc;
+        const C2 a      = acc[c];
+        acc[c]          = C2{fma2(a.re, bc2(ms), fma2(xv[c].re, fr, mul2(xv[c].im, nf))),
+                    fma2(a.im, bc2(ms), fma2(xv[c].im, fr, mul2(xv[c].re, fi)))};
+    }
+}
+// r -= alpha acc on the FP32 residual staged in the two epilogue slots (written
+// back to rw), |r|^2 added to dre
+template <int P, int NL>
+__device__ __forceinline__ void pk_cg_residual(const C2 acc[12], const double* alpha, float4* rw, int ss, int j,
+                                               const uint4* s8, const uint4* s9, float2& dre)
+{
+    const float ar = (float)alpha[0], ai = (float)alpha[1];
+#pragma unroll
+    for (int c = 0; c < 12; ++c) {
+        C2 r        = c2_from(as_f4(residual_chunk<P, NL>(s8, s9, c)), false);
+        const C2 v  = acc[c];
+        r.re        = fma2(v.re, bc2(-ar), fma2(v.im, bc2(ai), r.re));
+        r.im        = fma2(v.im, bc2(-ar), fma2(v.re, bc2(-ai), r.im));
+        __stcs(rw + (size_t)c * ss + j, c2_to(r));
+        dre         = fma2(r.re, r.re, fma2(r.im, r.im, dre));
+    }
+}
+// x += alpha p: p staged at s8, the FP32 x in the rest of the two epilogue slots
+template <int P, int NL>
+__device__ __forceinline__ void pk_cg_solution(const double* alpha, float4* xw, int ss, int j, const uint4* s8,
+                                               const uint4* s9)
+{
+    const float ar = (float)alpha[0], ai = (float)alpha[1];
+    C2 pv[12];
+    float2 ps;
+    staged_operand<P>(s8, pv, &ps);
+    const float2 cr = mul2(bc2(ar), ps), ci = mul2(bc2(ai), ps), nci = mul2(bc2(-ai), ps);
+#pragma unroll
+    for (int c = 0; c < 12; ++c) {
+        C2 xv = c2_from(as_f4(residual_chunk<P, NL>(s8, s9, c)), false);
+        xv.re = fma2(pv[c].re, cr, fma2(pv[c].im, nci, xv.re));
+        xv.im = fma2(pv[c].im, cr, fma2(pv[c].re, ci, xv.im));
+        __stcs(xw + (size_t)c * ss + j, c2_to(xv));
+    }
+}
+// |acc|^2 added to dre
+__device__ __forceinline__ void pk_self_dot(const C2 acc[12], float2& dre)
+{
+#pragma unroll
+    for (int c = 0; c < 12; ++c) dre = fma2(acc[c].re, acc[c].re, fma2(acc[c].im, acc[c].im, dre));
+}
+
 template <int P, int NL, int EPI, int DOT, int PH, int CFG>
 __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, CFG>::MINB) pdslash_kernel(const PkParams<P> prm)
 {
     using S = PkStage<P, NL, CFG>;
-    static_assert(S::STAGES == 2 || S::STAGES == 3, "the prologue below issues one or two stages");
     static_assert(DOT != DOT_XUPD || EPI != EPI_AXPY, "the solution update shares the EPI_AXPY operand slot");
     constexpr bool RED = DOT != DOT_NONE && DOT != DOT_XUPD;  // a reduction is fused
     pdl_enter();
@@ -524,133 +705,27 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, CFG>::MINB) pdslash
     float2 dre = bc2(0.f), dim = bc2(0.f), dq = bc2(0.f);
 
     if (j < g.H) {
-        // coordinates of slot j (site 0 at time t < NT/2; site 1 at t + NT/2)
-        const unsigned r1 = fdiv((unsigned)j, g.div_nsh);
-        const int xh      = j - (int)r1 * g.nsh;
-        const unsigned r2 = fdiv(r1, g.div_ns);
-        const int y       = (int)r1 - (int)r2 * g.ns;
-        const int t       = (int)fdiv(r2, g.div_ns);
-        const int z       = (int)r2 - t * g.ns;
-        const int x       = 2 * xh + ((prm.out_parity + y + z + t) & 1);
-        const int yzt     = j - xh;
-        const int ss      = g.ss;
-
-        const int po          = prm.out_parity;
-        const size_t grp      = (size_t)pk_link_bytes<P, NL>() * ss;
-        const char* gb        = static_cast<const char*>(prm.gauge);
-        const char* fwd_links = gb + (size_t)(po * 4) * grp;
-        const char* bwd_links = gb + (size_t)((1 - po) * 4) * grp;
-
-        // neighbour slot and link slot of the 8 hops (q = 2 mu + back); across
-        // the fold in time the neighbour slot holds the pair swapped
-        const bool fold_f = t + 1 == g.nt2, fold_b = t == 0;
-        const int base    = j - g.vs_h * t;
-        int nb[8];
-        nb[0]        = fold_f ? base : j + g.vs_h;
-        nb[1]        = fold_b ? base + g.vs_h * (g.nt2 - 1) : j - g.vs_h;
-        const int xp = x + 1 == g.ns ? 0 : x + 1, xm = x == 0 ? g.ns - 1 : x - 1;
-        nb[2]        = (xp >> 1) + yzt;
-        nb[3]        = (xm >> 1) + yzt;
-        const int row = g.nsh, pl = g.nsh * g.ns;
-        nb[4]         = y + 1 == g.ns ? j - (g.ns - 1) * row : j + row;
-        nb[5]         = y == 0 ? j + (g.ns - 1) * row : j - row;
-        nb[6]         = z + 1 == g.ns ? j - (g.ns - 1) * pl : j + pl;
-        nb[7]         = z == 0 ? j + (g.ns - 1) * pl : j - pl;
-
-        // stage q: hops 0..7, then the epilogue operands x (q = 8) and y (q = 9);
-        // every index below is a compile-time constant
-        auto issue = [&](auto qc) {
-            constexpr int q = decltype(qc)::value;
-            uint4* st       = mine + (size_t)((q % S::STAGES) * S::CH) * PK_THREADS;
-            if constexpr (q < 8) {
-                constexpr bool back = q & 1;
-                stage_spinor<P>(st, rr.in, rr.in_norm, ss, nb[q]);
-                // temporal gauge: the T links between inner slices are the identity
-                if (PH != PH_TG || q >= 2 || (back ? fold_b : fold_f))
-                    stage_link<P, NL>(st, (back ? bwd_links : fwd_links) + (size_t)(q >> 1) * grp, ss,
-                                      back ? nb[q] : j);
-            } else if constexpr (q == 8) {
+        const int ss = g.ss;
+        C2 acc[12];
+        pk_stencil<P, NL, PH, S>(acc, prm, rr.in, rr.in_norm, prm.out_parity, j, mine, [&](auto qc, uint4* st) {
+            if constexpr (decltype(qc)::value == 8) {
                 if (EPI == EPI_AXPY || DOT == DOT_XUPD) stage_spinor<P>(st, rr.x, rr.x_norm, ss, j);
                 if (DOT == DOT_CGR || DOT == DOT_XUPD) stage_residual<P, NL, 8>(st, rr.y, ss, j);
             } else {
                 if (DOT == DOT_Y) stage_spinor<P>(st, rr.y, rr.y_norm, ss, j);
                 if (DOT == DOT_CGR || DOT == DOT_XUPD) stage_residual<P, NL, 9>(st, rr.y, ss, j);
             }
-            cp_commit();
-        };
+        });
 
-        C2 acc[12];
-#pragma unroll
-        for (int c = 0; c < 12; ++c) acc[c] = C2{bc2(0.f), bc2(0.f)};
-
-        auto step = [&](auto hc) {
-            constexpr int h = decltype(hc)::value;
-            if constexpr (h + S::STAGES - 1 <= 9)
-                issue(std::integral_constant<int, h + S::STAGES - 1>{});
-            else
-                cp_commit();
-            cp_wait<S::STAGES - 1>();
-            const uint4* st = mine + (size_t)((h % S::STAGES) * S::CH) * PK_THREADS;
-            constexpr int mu = h >> 1;
-            constexpr bool back = h & 1;
-            if constexpr (mu == 0 && PH == PH_TG) {
-                if (back ? fold_b : fold_f)
-                    pk_hop_tg_fold<P, NL, back>(acc, prm, st);
-                else
-                    pk_hop_id<P, back>(acc, st, 1.0f);
-            } else if constexpr (mu == 0) {
-                if (back ? fold_b : fold_f)
-                    pk_hop_ph<P, NL, 0, back, true, PH>(acc, prm, st);
-                else
-                    pk_hop_ph<P, NL, 0, back, false, PH>(acc, prm, st);
-            } else {
-                pk_hop_ph<P, NL, mu, back, false, PH>(acc, prm, st);
-            }
-        };
-        issue(std::integral_constant<int, 0>{});
-        if constexpr (S::STAGES > 2) issue(std::integral_constant<int, 1>{});
-        step(std::integral_constant<int, 0>{});
-        step(std::integral_constant<int, 1>{});
-        step(std::integral_constant<int, 2>{});
-        step(std::integral_constant<int, 3>{});
-        step(std::integral_constant<int, 4>{});
-        step(std::integral_constant<int, 5>{});
-        step(std::integral_constant<int, 6>{});
-        step(std::integral_constant<int, 7>{});
-        if constexpr (S::STAGES == 2) issue(std::integral_constant<int, 9>{});
-        cp_wait<0>();
-
-        // epilogue on h = scale * acc (scale = -kappa, times the FP16 scales)
-        const float sc = (float)prm.c.scale;
-        if (EPI == EPI_PLAIN) {
-#pragma unroll
-            for (int c = 0; c < 12; ++c) acc[c] = C2{mul2(acc[c].re, bc2(sc)), mul2(acc[c].im, bc2(sc))};
-        } else if (EPI == EPI_DIAG) {
-#pragma unroll
-            for (int c = 0; c < 12; ++c) {
-                const float fr = (float)(c < 6 ? prm.e.f1re : prm.e.f2re) * sc;
-                const float fi = (float)(c < 6 ? prm.e.f1im : prm.e.f2im) * sc;
-                const C2 a     = acc[c];
-                acc[c]         = C2{fma2(a.re, bc2(fr), mul2(a.im, bc2(-fi))), fma2(a.im, bc2(fr), mul2(a.re, bc2(fi)))};
-            }
-        } else if (EPI == EPI_AXPY) {
-            // [g5] (f x - sc acc); FP16 x as exact integers q with the per-site
-            // scale folded into f, the sign of g5 folded into the coefficients
-            C2 xv[12];
-            float2 xs;
-            staged_operand<P>(mine + (size_t)((8 % S::STAGES) * S::CH) * PK_THREADS, xv, &xs);
-#pragma unroll
-            for (int c = 0; c < 12; ++c) {
-                const float gs  = (prm.e.gamma5 && c >= 6) ? -1.0f : 1.0f;
-                const float2 fr = mul2(bc2(gs * (float)(c < 6 ? prm.e.f1re : prm.e.f2re)), xs);
-                const float2 fi = mul2(bc2(gs * (float)(c < 6 ? prm.e.f1im : prm.e.f2im)), xs);
-                const float2 nf = mul2(bc2(-gs * (float)(c < 6 ? prm.e.f1im : prm.e.f2im)), xs);
-                const float ms  = -gs * sc;
-                const C2 a      = acc[c];
-                acc[c]          = C2{fma2(a.re, bc2(ms), fma2(xv[c].re, fr, mul2(xv[c].im, nf))),
-                            fma2(a.im, bc2(ms), fma2(xv[c].im, fr, mul2(xv[c].re, fi)))};
-            }
-        }
+        const float sc  = (float)prm.c.scale;
+        const uint4* s8 = mine + (size_t)((8 % S::STAGES) * S::CH) * PK_THREADS;
+        const uint4* s9 = mine + (size_t)((9 % S::STAGES) * S::CH) * PK_THREADS;
+        if (EPI == EPI_PLAIN)
+            pk_epi_plain(acc, sc);
+        else if (EPI == EPI_DIAG)
+            pk_epi_diag(acc, prm.e, sc);
+        else
+            pk_epi_axpy<P>(acc, prm.e, sc, s8);
         if (DOT != DOT_CGR) {
             if constexpr (P == 16)
                 SlotF16::store(rr.out, rr.out_norm, ss, j, acc);
@@ -658,24 +733,13 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, CFG>::MINB) pdslash
                 SlotF32::store(rr.out, ss, j, acc);
         }
 
-        if (DOT == DOT_CGR) {  // r -= alpha out (r FP32, passed as y, staged in the ring), |r|^2
-            const float ar = (float)rr.sc->alpha[0], ai = (float)rr.sc->alpha[1];
-            float4* rw     = static_cast<float4*>(const_cast<void*>(rr.y));
-            const uint4* s8 = mine + (size_t)((8 % S::STAGES) * S::CH) * PK_THREADS;
-            const uint4* s9 = mine + (size_t)((9 % S::STAGES) * S::CH) * PK_THREADS;
-#pragma unroll
-            for (int c = 0; c < 12; ++c) {
-                C2 r        = c2_from(as_f4(residual_chunk<P, NL>(s8, s9, c)), false);
-                const C2 v  = acc[c];
-                r.re        = fma2(v.re, bc2(-ar), fma2(v.im, bc2(ai), r.re));
-                r.im        = fma2(v.im, bc2(-ar), fma2(v.re, bc2(-ai), r.im));
-                __stcs(rw + (size_t)c * ss + j, c2_to(r));
-                dre         = fma2(r.re, r.re, fma2(r.im, r.im, dre));
-            }
+        float4* yw = static_cast<float4*>(const_cast<void*>(rr.y));  // the field a fused CG update changes
+        if (DOT == DOT_CGR) {
+            pk_cg_residual<P, NL>(acc, rr.sc->alpha, yw, ss, j, s8, s9, dre);
         } else if (DOT == DOT_Y) {  // conj(y) out, FP16 y as integers times the per-site scale
             C2 yv[12];
             float2 ys;
-            staged_operand<P>(mine + (size_t)((9 % S::STAGES) * S::CH) * PK_THREADS, yv, &ys);
+            staged_operand<P>(s9, yv, &ys);
 #pragma unroll
             for (int c = 0; c < 12; ++c) {
                 dre = fma2(yv[c].re, acc[c].re, fma2(yv[c].im, acc[c].im, dre));
@@ -686,24 +750,9 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, CFG>::MINB) pdslash
             dim = mul2(dim, ys);
             dq  = mul2(dq, ys);
         } else if (DOT == DOT_SELF) {
-#pragma unroll
-            for (int c = 0; c < 12; ++c) dre = fma2(acc[c].re, acc[c].re, fma2(acc[c].im, acc[c].im, dre));
-        } else if (DOT == DOT_XUPD) {  // x += alpha p (x FP32, passed as y; p passed as x; both staged)
-            const float ar  = (float)rr.sc->alpha[0], ai = (float)rr.sc->alpha[1];
-            float4* xw      = static_cast<float4*>(const_cast<void*>(rr.y));
-            const uint4* s8 = mine + (size_t)((8 % S::STAGES) * S::CH) * PK_THREADS;
-            const uint4* s9 = mine + (size_t)((9 % S::STAGES) * S::CH) * PK_THREADS;
-            C2 pv[12];
-            float2 ps;
-            staged_operand<P>(s8, pv, &ps);
-            const float2 cr = mul2(bc2(ar), ps), ci = mul2(bc2(ai), ps), nci = mul2(bc2(-ai), ps);
-#pragma unroll
-            for (int c = 0; c < 12; ++c) {
-                C2 xv = c2_from(as_f4(residual_chunk<P, NL>(s8, s9, c)), false);
-                xv.re = fma2(pv[c].re, cr, fma2(pv[c].im, nci, xv.re));
-                xv.im = fma2(pv[c].im, cr, fma2(pv[c].re, ci, xv.im));
-                __stcs(xw + (size_t)c * ss + j, c2_to(xv));
-            }
+            pk_self_dot(acc, dre);
+        } else if (DOT == DOT_XUPD) {
+            pk_cg_solution<P, NL>(rr.sc->alpha, yw, ss, j, s8, s9);
         }
     }
     if (RED) {  // one partial per tile, in tile order

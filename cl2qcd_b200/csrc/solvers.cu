@@ -549,7 +549,7 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
     if (!rc) rc = gauge_ensure(const_cast<c2q_gauge*>(g), gk64);
     if (rc) return rc;
     SolverScalars* dsc = nullptr;
-    C2Q_CUDA(ctx, cudaMallocAsync(&dsc, n * sizeof(SolverScalars), ctx->stream));
+    C2Q_CUDA(ctx, cudaMallocAsync(&dsc, n * sizeof(SolverScalars) + pcg_ctl_bytes(), ctx->stream));
     struct Free {
         c2q_ctx* c;
         void* q;
@@ -675,8 +675,44 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
         for (int k = 0; k < n; ++k)
             if (S[k].active) act.push_back(k);
         if (act.empty()) break;
-        hist[iter % 4] = act;
-        if (graphs && iter > 0) {
+        hist[iter % 4]   = act;
+        const bool whole = (int)act.size() <= whole_most;
+        if (whole) {
+            PcgBatch C;
+            PcgResult R;
+            C.n = (int)act.size();
+            for (int i = 0; i < C.n; ++i) {
+                const int k = act[i];
+                C.p[i]      = p[k];
+                C.t1[i]     = t1[k];
+                C.t2[i]     = t2[k];
+                C.rs[i]     = rs[k];
+                C.xs[i]     = xs[k];
+                C.sc[i]     = dsc + k;
+                C.thr[i]    = S[k].thr;
+                C.maxrr[i]  = S[k].maxrr;
+                C.skip[i]   = iter - 1 <= S[k].skip_upto;
+            }
+            C.kappa  = kappa;
+            C.mubar  = mubar;
+            C.delta  = delta;
+            C.action = action;
+            C.first  = iter == 0;
+            C.iters  = P->cgmax - iter;
+            C.ctl    = dsc + n;
+            rc       = pcg_run(ctx, g, gk, C, &R);
+            if (rc) return rc;
+            iter += R.iters - 1;  // the last iteration done
+            hist[(iter + 3) % 4] = act;
+            for (int i = 0; i < C.n; ++i) {
+                RhsState& s = S[act[i]];
+                s.sweeps += per_apply * R.iters;
+                s.maxrr       = R.maxrr[i];
+                double* slot  = ctx->batch_ring + (size_t)((iter + 3) % 4) * PK_MAX_RHS * 4 + 4 * act[i];
+                slot[0]       = R.judged[i];
+                memcpy(slot + 3, &R.flag[i], sizeof(int));
+            }
+        } else if (graphs && iter > 0) {
             if (graph.set != act) {
                 graph.reset();
                 cudaGraph_t gr     = nullptr;
@@ -702,12 +738,14 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
             rc = body(act, iter > 0);
             if (rc) return rc;
         }
-        for (int k : act) S[k].sweeps += per_apply;
-        rc = ring_push(ctx, iter, ctx->batch_ring_dev + (size_t)(iter % 4) * PK_MAX_RHS * 4, &dsc[0].resid,
-                       sizeof(SolverScalars), 4 * sizeof(double), n);
-        if (rc) return rc;
+        if (!whole) {
+            for (int k : act) S[k].sweeps += per_apply;
+            rc = ring_push(ctx, iter, ctx->batch_ring_dev + (size_t)(iter % 4) * PK_MAX_RHS * 4, &dsc[0].resid,
+                           sizeof(SolverScalars), 4 * sizeof(double), n);
+            if (rc) return rc;
+        }
         if (iter == 0) continue;
-        C2Q_CUDA(ctx, cudaEventSynchronize(ctx->ring_ev[(iter - 1) % 4]));
+        if (!whole) C2Q_CUDA(ctx, cudaEventSynchronize(ctx->ring_ev[(iter - 1) % 4]));
         const double* prev = ctx->batch_ring + (size_t)((iter - 1) % 4) * PK_MAX_RHS * 4;
         for (int k : hist[(iter - 1) % 4]) {
             RhsState& s = S[k];
@@ -723,6 +761,10 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
                 rc       = take_out(k, nullptr);  // keep what was gained
                 if (rc) return rc;
                 continue;
+    // Small lattices: the iterations up to the next decision in one launch
+    int whole_most = 0;
+    if (use_tg && fused) rc = pcg_capacity(ctx, PB, gk, x[0]->geom, &whole_most);
+    if (rc) return rc;
             }
             const double rn = std::sqrt(resid);
             if (rn > s.maxrr) s.maxrr = rn;
