@@ -252,7 +252,60 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
     double resid = std::numeric_limits<double>::quiet_NaN();
     bool force_refresh = false;
     double r2_confirmed = -1.0;  // true residual of the returned solution, when already computed
-    if (P->rel_tol > 0) {
+    if (pcg64_applies(ctx, op, g)) {
+        // Small lattices: everything between two refreshes in one launch.  With
+        // rel_tol every residual is judged, one iteration after its own as below,
+        // and a converged one confirmed by a true residual; else every
+        // resid_check_every-th, at once.
+        const bool lag = P->rel_tol > 0;
+        const int end  = std::max(P->cgmax, P->min_iter);
+        int skip_upto  = -1;
+        while (iter < end) {
+            Pcg64Solve S{x, rn, p, t1, t2, kappa, mubar, action};
+            if (iter % P->iter_refresh == 0 || force_refresh) {
+                force_refresh = false;
+                rc = apply_operator(ctx, op, rn, g, gk, x, kappa, mubar, action, t1, t2, DotSpec{}, &sweeps);
+                if (!rc) rc = saxpy_norm(ctx, rn, Cx{1, 0}, rn, b, FIN_CG_OMEGA, nullptr);
+                if (!rc) rc = copy_field(ctx, p, rn);
+                if (rc) return rc;
+                S.p_ready = 1;
+            }
+            S.iter0       = iter;
+            S.iters       = std::min(end, (iter / P->iter_refresh + 1) * P->iter_refresh) - iter;
+            S.min_iter    = P->min_iter;
+            S.lag         = lag;
+            S.skip        = iter - 1 <= skip_upto;
+            S.check_every = P->resid_check_every;
+            S.thr         = thr;
+            Pcg64Result R;
+            rc = pcg64_run(ctx, g, gk, S, &R);
+            if (rc) return rc;
+            sweeps += 4 * R.iters;
+            iter += R.iters - 1;  // the last iteration done
+            if (R.stop || R.judged == R.judged) resid = R.judged;
+            if (R.stop) {
+                if (resid != resid) {
+                    status = C2Q_SOLVER_STUCK;
+                    break;
+                }
+                if (!lag) {
+                    status = iter;
+                    break;
+                }
+                double r2t = 0;
+                rc = true_residual(ctx, op, g, x, b, kappa, mubar, action, t2, t1, v, &r2t, &sweeps);
+                if (rc) return rc;
+                if (r2t <= P->rel_tol * P->rel_tol * b2 || (P->prec > 0 && r2t < P->prec)) {
+                    status       = iter;
+                    r2_confirmed = r2t;
+                    break;
+                }
+                force_refresh = true;  // the iterated residual drifted: restart from the true residual
+                skip_upto     = iter;
+            }
+            ++iter;
+        }
+    } else if (P->rel_tol > 0) {
         // True-residual target: residual monitored every iteration through the
         // pinned ring (no host round trip per iteration); a converged iterated
         // residual is confirmed by an FP64 true residual, else CG restarts from it.
@@ -670,6 +723,10 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
     // and applies its decisions after iteration k.
     std::vector<int> hist[4], act;
     int iter = 0;
+    // Small lattices: the iterations up to the next decision in one launch
+    int whole_most = 0;
+    if (use_tg && fused) rc = pcg_capacity(ctx, PB, gk, x[0]->geom, &whole_most);
+    if (rc) return rc;
     for (iter = 0; iter < P->cgmax; ++iter) {
         act.clear();
         for (int k = 0; k < n; ++k)
@@ -761,10 +818,6 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
                 rc       = take_out(k, nullptr);  // keep what was gained
                 if (rc) return rc;
                 continue;
-    // Small lattices: the iterations up to the next decision in one launch
-    int whole_most = 0;
-    if (use_tg && fused) rc = pcg_capacity(ctx, PB, gk, x[0]->geom, &whole_most);
-    if (rc) return rc;
             }
             const double rn = std::sqrt(resid);
             if (rn > s.maxrr) s.maxrr = rn;

@@ -1,0 +1,99 @@
+"""GPU: the cooperative CG iterations of small lattices (pcg.cuh, pcg64.cu) against the
+per-launch iterations, which per-launch profiling selects, and the oracle's operator.
+
+Lattices at the edges of the tiles (128 slots of two sites; 32 sites): one tile, a whole
+number of tiles, a ragged last tile.  The mixed-precision iterations are the same
+arithmetic in the same order: bitwise.  The FP64 ones differ by rounding: the same
+iteration count, and solutions of two solves to the same residual."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+LATTICES = [(4, 4), (4, 8), (6, 12), (10, 8), (8, 16)]
+
+
+def _solve(c2q, system, L, gf, srcs, params, add, action="twistedmass", per_launch=False):
+    bs = [c2q.Spinorfield_eo(system, L, s) for s in srcs]
+    xs = [c2q.Spinorfield_eo(system, L) for _ in srcs]
+    reps = []
+    system.lib.c2q_ctx_profile(system.h, int(per_launch))
+    try:
+        c2q.host.cg_multi(xs, c2q.host.QplusQminus_eo(action), gf, bs, params, add, reps)
+    finally:
+        system.lib.c2q_ctx_profile(system.h, 0)
+    return [x.dump() for x in xs], reps
+
+
+@pytest.mark.parametrize("ns,nt", LATTICES)
+@pytest.mark.parametrize("precision,rec12,action", [(16, True, "twistedmass"), (16, False, "wilson"),
+                                                    (32, True, "wilson"), (32, False, "twistedmass")])
+@pytest.mark.parametrize("n", [1, 3])
+def test_mixed_iterations_bitwise(port, system, O, ns, nt, precision, rec12, action, n):
+    import cl2qcd_b200 as c2q
+    port.set_lattice(ns, nt, 1.0, 0.0)
+    L = c2q.Lattice(ns, nt, 1.0, 0.0)
+    g = c2q.host.generate_gaugefield(L, 0.3, 11)
+    gf = c2q.Gaugefield(system, L, g)
+    srcs = [c2q.host.generate_source(L.seo, "z2" if k else "gaussian", 40 + k) for k in range(n)]
+    kappa, mubar = (0.12, 0.0) if action == "wilson" else (0.14, 2 * 0.14 * 0.05)
+    add = c2q.AdditionalParameters(kappa, mubar)
+    P = c2q.SolverParameters(solver="cg", prec=0.0, rel_tol=1e-10, cgmax=5000, precision=precision, use_rec12=rec12)
+    xa, ra = _solve(c2q, system, L, gf, srcs, P, add, action)
+    xb, rb = _solve(c2q, system, L, gf, srcs, P, add, action, per_launch=True)
+    for k in range(n):
+        assert ra[k]["iterations"] == rb[k]["iterations"]
+        assert ra[k]["reliable_updates"] == rb[k]["reliable_updates"]
+        assert ra[k]["dslash_applications"] == rb[k]["dslash_applications"]
+        assert np.array_equal(xa[k], xb[k])
+        r = port.apply(O.OP_QPQM_EO, xa[k], g, kappa, mubar, action=O.WILSON if action == "wilson" else O.TWISTEDMASS)
+        assert np.linalg.norm(r - srcs[k]) / np.linalg.norm(srcs[k]) <= 1.5e-10
+
+
+@pytest.mark.parametrize("ns,nt", LATTICES + [(6, 10)])
+@pytest.mark.parametrize("rec12,action", [(False, "twistedmass"), (True, "wilson")])
+@pytest.mark.parametrize("mode", ["rel_tol", "refresh", "prec"])
+def test_fp64_iterations(port, system, O, ns, nt, rec12, action, mode):
+    import cl2qcd_b200 as c2q
+    port.set_lattice(ns, nt, 1.0, 0.0)
+    L = c2q.Lattice(ns, nt, 1.0, 0.0)
+    g = c2q.host.generate_gaugefield(L, 0.3, 12)
+    gf = c2q.Gaugefield(system, L, g)
+    src = c2q.host.generate_source(L.seo, "gaussian", 50)
+    kappa, mubar = (0.12, 0.0) if action == "wilson" else (0.14, 2 * 0.14 * 0.05)
+    add = c2q.AdditionalParameters(kappa, mubar)
+    kw = {"rel_tol": dict(prec=0.0, rel_tol=1e-10), "refresh": dict(prec=0.0, rel_tol=1e-10, iter_refresh=7),
+          "prec": dict(prec=1e-20 * float(np.sum(src ** 2)), resid_check_every=3)}[mode]
+    P = c2q.SolverParameters(solver="cg", cgmax=5000, precision=64, use_rec12=rec12, **kw)
+    xa, ra = _solve(c2q, system, L, gf, [src], P, add, action)
+    xb, rb = _solve(c2q, system, L, gf, [src], P, add, action, per_launch=True)
+    assert abs(ra[0]["iterations"] - rb[0]["iterations"]) <= (3 if mode == "prec" else 1)
+    assert ra[0]["true_resid_rel"] <= 1e-10
+    r = port.apply(O.OP_QPQM_EO, xa[0], g, kappa, mubar, action=O.WILSON if action == "wilson" else O.TWISTEDMASS)
+    assert np.linalg.norm(r - src) / np.linalg.norm(src) <= 1.01e-10
+    assert rel_l2(xa[0], xb[0]) <= 1e-8
+
+
+@pytest.mark.parametrize("precision", [64, 32, 16])
+def test_limits_and_nan(system, precision):
+    """The iteration limit and a residual that is no number end the solve as before."""
+    import cl2qcd_b200 as c2q
+    L = c2q.Lattice(6, 8, 1.0, 0.0)
+    gf = c2q.Gaugefield(system, L, c2q.host.generate_gaugefield(L, 0.3, 13))
+    add = c2q.AdditionalParameters(0.14, 2 * 0.14 * 0.05)
+    src = c2q.host.generate_source(L.seo, "z2", 51)
+    for cgmax in (1, 2, 9):
+        x, b = c2q.Spinorfield_eo(system, L), c2q.Spinorfield_eo(system, L, src)
+        rep = {}
+        with pytest.raises(c2q.SolverDidNotSolve):
+            c2q.host.cg(x, c2q.host.QplusQminus_eo(), gf, b,
+                        c2q.SolverParameters(solver="cg", prec=0.0, rel_tol=1e-10, cgmax=cgmax, precision=precision),
+                        add, rep)
+        assert rep["iterations"] == cgmax and np.isfinite(rep["true_resid_rel"])
+    src[3, 5] = np.nan
+    x, b = c2q.Spinorfield_eo(system, L), c2q.Spinorfield_eo(system, L, src)
+    with pytest.raises((c2q.SolverStuck, c2q.SolverDidNotSolve)):
+        c2q.host.cg(x, c2q.host.QplusQminus_eo(), gf, b,
+                    c2q.SolverParameters(solver="cg", prec=0.0, rel_tol=1e-10, cgmax=50, precision=precision), add)
