@@ -43,6 +43,9 @@ struct c2q_ctx {
     // staging buffer for AoS host <-> device transfers
     void* staging          = nullptr;
     size_t staging_cap     = 0;
+    // ring of pinned buffers between pageable host arrays and the device (hostcopy.cu)
+    void* hc_ring        = nullptr;
+    cudaEvent_t hc_ev[4] = {};
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t ring_ev[4] = {};  // residual ring of the pipelined solvers
     // The pipelined solvers copy each iteration's residual into ring_dev on the
@@ -192,6 +195,12 @@ int tg_to_inner(c2q_ctx* ctx, const c2q_gauge* g, c2q_spinor_eo* out, const c2q_
 int tg_accumulate(c2q_ctx* ctx, const c2q_gauge* g, c2q_spinor_eo* x, c2q_spinor_eo* xs, const c2q_spinor_eo* p,
                   const SolverScalars* sc);
 int ensure_staging(c2q_ctx* ctx, size_t bytes);
+// Host array -> device and back on the context's stream, at PCIe rate from and into
+// pageable memory too (hostcopy.cu).  copy_to_host returns when the array is
+// filled; copy_to_device may still be in flight, but has read a pageable array
+// (a pinned one must stay valid until the stream has passed the copy).
+int copy_to_device(c2q_ctx* ctx, void* dev, const void* host, size_t bytes);
+int copy_to_host(c2q_ctx* ctx, void* host, const void* dev, size_t bytes);
 // Small copies (multiples of 4 bytes) between device memory and the device alias
 // of a pinned host buffer, by a one-block kernel on the context's stream:
 // `height` rows of `width` bytes, rows `dpitch` / `spitch` bytes apart.

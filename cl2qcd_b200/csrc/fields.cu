@@ -808,6 +808,9 @@ C2Q_EXPORT int c2q_ctx_destroy(c2q_ctx* ctx)
     cudaFree(ctx->red_result);
     cudaFree(ctx->scalars);
     cudaFree(ctx->staging);
+    if (ctx->hc_ring) cudaFreeHost(ctx->hc_ring);
+    for (auto e : ctx->hc_ev)
+        if (e) cudaEventDestroy(e);
     if (ctx->host_pinned) cudaFreeHost(ctx->host_pinned);
     profile_recycle(ctx);
     for (auto e : ctx->event_pool) cudaEventDestroy(e);
@@ -922,7 +925,8 @@ C2Q_EXPORT int c2q_gauge_upload(c2q_gauge* g, const double* aos)
     const size_t bytes = (size_t)4 * vol * 18 * sizeof(double);
     int rc           = ensure_staging(ctx, bytes);
     if (rc) return rc;
-    C2Q_CUDA(ctx, cudaMemcpyAsync(ctx->staging, aos, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    rc = copy_to_device(ctx, ctx->staging, aos, bytes);
+    if (rc) return rc;
     const long long n = 4LL * vol;
     gauge_import_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(
         (const double2*)ctx->staging, (double2*)g->store[G64].data, g->geom, vol);
@@ -950,9 +954,7 @@ C2Q_EXPORT int c2q_gauge_download(const c2q_gauge* g, double* aos)
         (double2*)ctx->staging, (const double2*)g->store[G64].data, g->geom, vol);
     ctx->launches++;
     C2Q_CUDA(ctx, cudaGetLastError());
-    C2Q_CUDA(ctx, cudaMemcpyAsync(aos, ctx->staging, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return C2Q_OK;
+    return copy_to_host(ctx, aos, ctx->staging, bytes);
 }
 
 // ---------------------------------------------------------------- spinors
@@ -985,8 +987,9 @@ C2Q_EXPORT int c2q_spinor_eo_destroy(c2q_spinor_eo* f)
     return C2Q_OK;
 }
 
+// (wait: a transfer on the context's stream that the caller waits for, else enqueued on `stream`)
 static int aos_transfer(c2q_spinor_eo* f, double* host_dst, const double* host_src, int mode, int par,
-                        const double* dev_src_full, cudaStream_t stream = nullptr)
+                        const double* dev_src_full, bool wait = true, cudaStream_t stream = nullptr)
 {
     c2q_ctx* ctx       = f->ctx;
     cudaStream_t st    = stream ? stream : ctx->stream;
@@ -1005,7 +1008,12 @@ static int aos_transfer(c2q_spinor_eo* f, double* host_dst, const double* host_s
         if (host_src) {
             int rc = ensure_staging(ctx, bytes);
             if (rc) return rc;
-            C2Q_CUDA(ctx, cudaMemcpyAsync(ctx->staging, host_src, bytes, cudaMemcpyHostToDevice, st));
+            if (wait) {
+                rc = copy_to_device(ctx, ctx->staging, host_src, bytes);
+                if (rc) return rc;
+            } else {
+                C2Q_CUDA(ctx, cudaMemcpyAsync(ctx->staging, host_src, bytes, cudaMemcpyHostToDevice, st));
+            }
             A.aos = static_cast<double*>(ctx->staging);
         } else {
             A.aos = const_cast<double*>(dev_src_full);
@@ -1018,9 +1026,8 @@ static int aos_transfer(c2q_spinor_eo* f, double* host_dst, const double* host_s
         soa_to_aos_kernel<<<blocks, 256, 0, st>>>(A);
         ctx->launches++;
         C2Q_CUDA(ctx, cudaGetLastError());
-        if (host_dst) {
-            C2Q_CUDA(ctx, cudaMemcpyAsync(host_dst, ctx->staging, bytes, cudaMemcpyDeviceToHost, st));
-        }
+        if (host_dst && wait) return copy_to_host(ctx, host_dst, ctx->staging, bytes);
+        if (host_dst) C2Q_CUDA(ctx, cudaMemcpyAsync(host_dst, ctx->staging, bytes, cudaMemcpyDeviceToHost, st));
     }
     return C2Q_OK;
 }
@@ -1076,7 +1083,7 @@ C2Q_EXPORT int c2q_spinor_eo_upload_async(c2q_spinor_eo* f, const double* aos, v
     if (!f || !aos) return C2Q_BAD_ARG;
     if (f->prec != 64) return fail(f->ctx, C2Q_BAD_ARG, "asynchronous transfers take FP64 fields");
     const int rc = ensure_staging(f->ctx, (size_t)f->geom.seo * 24 * sizeof(double));
-    return rc ? rc : aos_transfer(f, nullptr, aos, 0, 0, nullptr, static_cast<cudaStream_t>(stream));
+    return rc ? rc : aos_transfer(f, nullptr, aos, 0, 0, nullptr, false, static_cast<cudaStream_t>(stream));
 }
 
 C2Q_EXPORT int c2q_spinor_eo_download_async(const c2q_spinor_eo* f, double* aos, void* stream)
@@ -1085,7 +1092,7 @@ C2Q_EXPORT int c2q_spinor_eo_download_async(const c2q_spinor_eo* f, double* aos,
     c2q_spinor_eo* ff = const_cast<c2q_spinor_eo*>(f);
     if (f->prec != 64) return fail(f->ctx, C2Q_BAD_ARG, "asynchronous transfers take FP64 fields");
     const int rc = ensure_staging(ff->ctx, (size_t)f->geom.seo * 24 * sizeof(double));
-    return rc ? rc : aos_transfer(ff, aos, nullptr, 0, 0, nullptr, static_cast<cudaStream_t>(stream));
+    return rc ? rc : aos_transfer(ff, aos, nullptr, 0, 0, nullptr, false, static_cast<cudaStream_t>(stream));
 }
 
 C2Q_EXPORT int c2q_spinor_eo_precision(const c2q_spinor_eo* f) { return f ? f->prec : C2Q_BAD_ARG; }
@@ -1253,8 +1260,8 @@ C2Q_EXPORT int c2q_convert_to_eoprec(c2q_spinor_eo* even, c2q_spinor_eo* odd, co
     const size_t bytes = (size_t)even->geom.seo * 2 * 24 * sizeof(double);
     int rc             = ensure_staging(ctx, bytes);
     if (rc) return rc;
-    C2Q_CUDA(ctx, cudaMemcpyAsync(ctx->staging, full, bytes, cudaMemcpyHostToDevice, ctx->stream));
-    rc = aos_transfer(even, nullptr, nullptr, 1, 0, (const double*)ctx->staging);
+    rc = copy_to_device(ctx, ctx->staging, full, bytes);
+    if (!rc) rc = aos_transfer(even, nullptr, nullptr, 1, 0, (const double*)ctx->staging);
     if (!rc) rc = aos_transfer(odd, nullptr, nullptr, 1, 1, (const double*)ctx->staging);
     if (rc) return rc;
     C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1283,9 +1290,7 @@ C2Q_EXPORT int c2q_convert_from_eoprec(double* full, const c2q_spinor_eo* even, 
         ctx->launches++;
         C2Q_CUDA(ctx, cudaGetLastError());
     }
-    C2Q_CUDA(ctx, cudaMemcpyAsync(full, ctx->staging, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return C2Q_OK;
+    return copy_to_host(ctx, full, ctx->staging, bytes);
 }
 
 // ---------------------------------------------------------------- explicit ops

@@ -274,7 +274,8 @@ C2Q_EXPORT int c2q_gaugemomenta_upload(c2q_gaugemomenta* m, const double* aos)
     const size_t bytes = (size_t)4 * vol * 8 * sizeof(double);
     int rc             = ensure_staging(ctx, bytes);
     if (rc) return rc;
-    C2Q_CUDA(ctx, cudaMemcpyAsync(ctx->staging, aos, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    rc = copy_to_device(ctx, ctx->staging, aos, bytes);
+    if (rc) return rc;
     const long long n = 4LL * vol;
     gm_import_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>((const double*)ctx->staging, m->data,
                                                                          m->geom, vol);
@@ -297,9 +298,7 @@ C2Q_EXPORT int c2q_gaugemomenta_download(const c2q_gaugemomenta* m, double* aos)
                                                                          vol);
     ctx->launches++;
     C2Q_CUDA(ctx, cudaGetLastError());
-    C2Q_CUDA(ctx, cudaMemcpyAsync(aos, ctx->staging, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return C2Q_OK;
+    return copy_to_host(ctx, aos, ctx->staging, bytes);
 }
 
 C2Q_EXPORT int c2q_gaugemomenta_squarenorm(const c2q_gaugemomenta* m, double* out)
