@@ -214,6 +214,12 @@ __device__ __forceinline__ void cp16(uint4* smem, const void* g)
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(g) : "memory");
 }
+// (kept in L1 for the other hops of the block that need the line)
+__device__ __forceinline__ void cp16_l1(uint4* smem, const void* g)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(g) : "memory");
+}
 __device__ __forceinline__ void cp8(uint4* smem, const void* g)
 {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -233,7 +239,7 @@ __device__ __forceinline__ void stage_spinor(uint4* st, const void* d, const flo
     const uint4* p  = static_cast<const uint4*>(d) + slot;
     constexpr int n = P == 16 ? 6 : 12;
 #pragma unroll
-    for (int c = 0; c < n; ++c) cp16(st + c * PK_THREADS, p + (size_t)c * ss);
+    for (int c = 0; c < n; ++c) cp16_l1(st + c * PK_THREADS, p + (size_t)c * ss);
     if (P == 16) cp8(st + 6 * PK_THREADS, reinterpret_cast<const float2*>(norm) + slot);
 }
 // link of `slot` of a (parity, mu) group -> chunks [SPC, CH)
