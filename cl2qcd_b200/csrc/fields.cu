@@ -1003,7 +1003,7 @@ static int aos_transfer(c2q_spinor_eo* f, double* host_dst, const double* host_s
     A.par    = par;
     A.ns     = f->geom.ns;
     A.nsh    = f->geom.nsh;
-    const int blocks = (A.n + 255) / 256;
+    const int blocks = (A.n + AOS_SITES - 1) / AOS_SITES;
     if (host_src || dev_src_full) {
         if (host_src) {
             int rc = ensure_staging(ctx, bytes);
@@ -1018,12 +1018,12 @@ static int aos_transfer(c2q_spinor_eo* f, double* host_dst, const double* host_s
         } else {
             A.aos = const_cast<double*>(dev_src_full);
         }
-        aos_to_soa_kernel<<<blocks, 256, 0, st>>>(A);
+        aos_to_soa_kernel<<<blocks, AOS_THREADS, 0, st>>>(A);
         ctx->launches++;
         C2Q_CUDA(ctx, cudaGetLastError());
     } else {
         A.aos = static_cast<double*>(ctx->staging);
-        soa_to_aos_kernel<<<blocks, 256, 0, st>>>(A);
+        soa_to_aos_kernel<<<blocks, AOS_THREADS, 0, st>>>(A);
         ctx->launches++;
         C2Q_CUDA(ctx, cudaGetLastError());
         if (host_dst && wait) return copy_to_host(ctx, host_dst, ctx->staging, bytes);
@@ -1286,7 +1286,7 @@ C2Q_EXPORT int c2q_convert_from_eoprec(double* full, const c2q_spinor_eo* even, 
         A.par    = par;
         A.ns     = f->geom.ns;
         A.nsh    = f->geom.nsh;
-        soa_to_aos_kernel<<<(A.n + 255) / 256, 256, 0, ctx->stream>>>(A);
+        soa_to_aos_kernel<<<(A.n + AOS_SITES - 1) / AOS_SITES, AOS_THREADS, 0, ctx->stream>>>(A);
         ctx->launches++;
         C2Q_CUDA(ctx, cudaGetLastError());
     }
