@@ -6,7 +6,7 @@
 #include <cstring>
 #include <vector>
 
-#include "blas.cuh"
+#include "blas_pk.cuh"
 #include "c2q_host.h"
 #include "dslash.cuh"
 
@@ -573,7 +573,10 @@ static int blas_typed(c2q_ctx* ctx, const BlasSpec& s, const c2q_spinor_eo* ref)
     }
     A.red         = red_args(ctx, s.fin);
     A.red.fin_arg = s.fin_arg;
-    C2Q_CUDA(ctx, launch_dep(ctx->pdl, blas_kernel<P>, dim3(blocks), dim3(BLAS_THREADS), 0, ctx->stream, A));
+    if constexpr (P == 64)
+        C2Q_CUDA(ctx, launch_dep(ctx->pdl, blas_kernel<P>, dim3(blocks), dim3(BLAS_THREADS), 0, ctx->stream, A));
+    else
+        C2Q_CUDA(ctx, launch_dep(ctx->pdl, blas_pk_kernel<P>, dim3(blocks), dim3(BLAS_PK_THREADS), 0, ctx->stream, A));
     ctx->launches++;
     C2Q_CUDA(ctx, cudaGetLastError());
     return C2Q_OK;
@@ -607,7 +610,8 @@ static int cg_update_typed(c2q_ctx* ctx, c2q_spinor_eo* x, c2q_spinor_eo* r, con
     A.sc = ctx->scalars;
     A.n = x->geom.seo;
     A.stride = x->geom.stride;
-    const int blocks = (A.n + BLAS_THREADS - 1) / BLAS_THREADS;
+    const int blocks = P == 64 ? (A.n + BLAS_THREADS - 1) / BLAS_THREADS
+                               : (A.n / 2 + BLAS_PK_THREADS - 1) / BLAS_PK_THREADS;
     int rc = ensure_partials(ctx, blocks);
     if (rc) return rc;
     A.red = red_args(ctx, FIN_CG_BETA);
@@ -656,8 +660,12 @@ template <int PO, int PI>
 static void convert_go(c2q_ctx* ctx, c2q_spinor_eo* out, const c2q_spinor_eo* in)
 {
     const int n = out->geom.seo;
-    convert_kernel<PO, PI><<<(n + BLAS_THREADS - 1) / BLAS_THREADS, BLAS_THREADS, 0, ctx->stream>>>(
-        sptr<PO>(out), sptr<PI>(in), n, out->geom.stride);
+    if constexpr (PO == 64 && PI == 64)
+        convert_kernel<PO, PI><<<(n + BLAS_THREADS - 1) / BLAS_THREADS, BLAS_THREADS, 0, ctx->stream>>>(
+            sptr<PO>(out), sptr<PI>(in), n, out->geom.stride);
+    else
+        convert_pk_kernel<PO, PI><<<(n / 2 + BLAS_PK_THREADS - 1) / BLAS_PK_THREADS, BLAS_PK_THREADS, 0, ctx->stream>>>(
+            sptr<PO>(out), sptr<PI>(in), n, out->geom.stride);
 }
 
 int launch_convert(c2q_ctx* ctx, c2q_spinor_eo* out, const c2q_spinor_eo* in)
