@@ -340,6 +340,16 @@ int apply_operator(c2q_ctx* ctx, int op, c2q_spinor_eo* out, const c2q_gauge* g,
                    const c2q_spinor_eo* in, double kappa, double mubar, int action, c2q_spinor_eo* tmp1,
                    c2q_spinor_eo* tmp2, const DotSpec& dot, int* sweeps);
 
+// Q+Q- in with the FP64 CG's vector updates fused in: alpha = omega / |Q- in|^2 after
+// the second sweep ((in, Q+Q- in) where Q+ is the adjoint of Q-), x += alpha in in
+// the third, r -= alpha Q+Q- in with |r|^2 -> beta in the last.
+int apply_qpqm_cg(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const c2q_spinor_eo* in, double kappa, double mubar,
+                  int action, c2q_spinor_eo* tmp1, c2q_spinor_eo* tmp2, c2q_spinor_eo* x, c2q_spinor_eo* r,
+                  int* sweeps);
+// every backward hop weight is the conjugate of the forward one (no real chemical
+// potential): Q+ is the adjoint of Q-
+bool adjoint_weights(const c2q_gauge* g);
+
 // Read back `n` doubles of device memory synchronously through pinned memory.
 int read_scalars(c2q_ctx* ctx, const double* dev, int n, double* host);
 

@@ -1,6 +1,7 @@
 // dslash.cuh -- the even-odd Wilson hopping term with fused twisted-mass
-// epilogues, for one output parity, one thread per output site, on the FP64
-// fields (the FP32 / FP16 fields use the paired-site kernel of pdslash.cuh).
+// epilogues: its spin projection and SU(3) products.  The sweeps over one output
+// parity are dslash64.cuh (FP64, one thread per site) and pdslash.cuh (FP32 / FP16,
+// one thread per slot of two sites).
 //
 // Computes, at every site x of the output parity,
 //   h(x) = sum_mu [ c_mu^+ (1 - g_mu) U_mu(x) psi(x+mu)
@@ -28,21 +29,6 @@
 #include "reduce.cuh"
 
 namespace c2q {
-
-template <int P>
-struct DslashParams {
-    SpinorPtr<P> out;
-    SpinorPtr<P> in;   // opposite-parity input field
-    SpinorPtr<P> x;    // EPI_AXPY: same-parity field multiplied by M_diag
-    SpinorPtr<P> y;    // DOT_Y partner (same parity as out)
-    const void* gauge; // [parity][mu][lane][stride]
-    Geom g;
-    HopCoef c;
-    EpiArgs e;
-    int out_parity;    // parity of the output sites: 0 = (x+y+z+t) even
-    RedArgs red;
-    int pdl;           // launched as a dependent launch (launch_dep)
-};
 
 // multiply by c in {1, -1, i, -i}, encoded as K = 0, 1, 2, 3
 template <int K, typename R>
@@ -141,133 +127,5 @@ __device__ __forceinline__ void hop_decoded(Cplx<R> acc[12], const Cplx<R> psi[1
 // link is the identity except the one leaving the last time slice, and the T
 // phase sits in the transformation), all hop coefficients are real.
 enum PhasePattern : int { PH_REAL = 0, PH_TCPLX = 1, PH_ANY = 2, PH_TG = 3 };
-
-// One hop: load the neighbour spinor and the link, weight by the hop phase.
-template <int P, int NL, int MU, bool BACK, int PH>
-__device__ __forceinline__ void do_hop(Cplx<typename Prec<P>::R> acc[12], const DslashParams<P>& prm,
-                                       const char* links, size_t link_idx, int i_nb)
-{
-    using R          = typename Prec<P>::R;
-    const Geom& g    = prm.g;
-    const size_t ls  = (size_t)g.stride;
-    const int d      = BACK ? 1 : 0;
-    const bool kreal = PH == PH_REAL ? true
-                       : PH == PH_TCPLX ? (MU != 0)
-                                        : (bool)((prm.c.real_mask >> (2 * MU + d)) & 1u);
-    Cplx<R> u[9];
-    Cplx<R> psi[12];
-    SpinorIO<P>::load(prm.in, g.stride, i_nb, psi);
-    LinkIO<P, NL>::load(links, ls, link_idx, u);
-    if (NL == 6) reconstruct_row2(u);
-    const Cplx<R> k = cmk<R>((R)prm.c.re[MU][d], (R)prm.c.im[MU][d]);
-    if (kreal)
-        hop_decoded<R, MU, BACK, true>(acc, psi, u, k);
-    else
-        hop_decoded<R, MU, BACK, false>(acc, psi, u, k);
-}
-
-template <int P, int NL, int MU, int PH>
-__device__ __forceinline__ void do_direction(Cplx<typename Prec<P>::R> acc[12], const DslashParams<P>& prm,
-                                             int i_fwd, int i_bwd, int i_site)
-{
-    const size_t ls       = (size_t)prm.g.stride;
-    const int po          = prm.out_parity;
-    constexpr size_t esz  = 16;  // one double2 per complex lane entry
-    const char* gbase     = static_cast<const char*>(prm.gauge);
-    const char* fwd_links = gbase + (size_t)((po * 4 + MU) * NL) * ls * esz;
-    const char* bwd_links = gbase + (size_t)(((1 - po) * 4 + MU) * NL) * ls * esz;
-    do_hop<P, NL, MU, false, PH>(acc, prm, fwd_links, (size_t)i_site, i_fwd);  // U_mu(x) psi(x+mu)
-    do_hop<P, NL, MU, true, PH>(acc, prm, bwd_links, (size_t)i_bwd, i_bwd);    // U_mu(x-mu)^dagger psi(x-mu)
-}
-
-template <int P, int NL, int EPI, int DOT, int PH>
-__global__ void __launch_bounds__(128) dslash_kernel(const DslashParams<P> prm)
-{
-    pdl_enter();
-    if (halted(prm.red)) return;  // a stopped device-driven solve: every block leaves
-    using R       = typename Prec<P>::R;
-    const Geom& g = prm.g;
-    const int i   = blockIdx.x * blockDim.x + threadIdx.x;
-    double dv[2]  = {0.0, 0.0};
-
-    if (i < g.seo) {
-        // coordinates of the output site carrying eo index i
-        int rest     = i / g.nsh;
-        const int xh = i - rest * g.nsh;
-        const int y  = rest % g.ns;
-        rest /= g.ns;
-        const int z  = rest % g.ns;
-        const int t  = rest / g.ns;
-        const int x  = 2 * xh + ((prm.out_parity + y + z + t) & 1);
-        const int yzt = g.nsh * (y + g.ns * (z + g.ns * t));
-
-        Cplx<R> acc[12];
-#pragma unroll
-        for (int k = 0; k < 12; ++k) acc[k] = cmk<R>(0, 0);
-
-        {  // T
-            const int tp = t + 1 == g.nt ? 0 : t + 1, tm = t == 0 ? g.nt - 1 : t - 1;
-            const int base = xh + g.nsh * (y + g.ns * z);
-            do_direction<P, NL, 0, PH>(acc, prm, base + g.vs_h * tp, base + g.vs_h * tm, i);
-        }
-        {  // X
-            const int xp = x + 1 == g.ns ? 0 : x + 1, xm = x == 0 ? g.ns - 1 : x - 1;
-            do_direction<P, NL, 1, PH>(acc, prm, (xp >> 1) + yzt, (xm >> 1) + yzt, i);
-        }
-        {  // Y
-            const int yp = y + 1 == g.ns ? 0 : y + 1, ym = y == 0 ? g.ns - 1 : y - 1;
-            const int zt = g.ns * (z + g.ns * t);
-            do_direction<P, NL, 2, PH>(acc, prm, xh + g.nsh * (yp + zt), xh + g.nsh * (ym + zt), i);
-        }
-        {  // Z
-            const int zp = z + 1 == g.ns ? 0 : z + 1, zm = z == 0 ? g.ns - 1 : z - 1;
-            do_direction<P, NL, 3, PH>(acc, prm, xh + g.nsh * (y + g.ns * (zp + g.ns * t)),
-                                   xh + g.nsh * (y + g.ns * (zm + g.ns * t)), i);
-        }
-
-        // the hopping sum is h = scale * acc (scale = -kappa, times the link dequantisation scale)
-        const R sc = (R)prm.c.scale;
-        if (EPI == EPI_PLAIN) {
-#pragma unroll
-            for (int k = 0; k < 12; ++k) acc[k] = cmk<R>(sc * acc[k].re, sc * acc[k].im);
-        } else if (EPI == EPI_DIAG) {
-            const Cplx<R> f1 = cmk<R>((R)prm.e.f1re * sc, (R)prm.e.f1im * sc);
-            const Cplx<R> f2 = cmk<R>((R)prm.e.f2re * sc, (R)prm.e.f2im * sc);
-#pragma unroll
-            for (int k = 0; k < 12; ++k) acc[k] = cmul(k < 6 ? f1 : f2, acc[k]);
-        } else if (EPI == EPI_AXPY) {
-            Cplx<R> xv[12];
-            SpinorIO<P>::load(prm.x, g.stride, i, xv);
-            const Cplx<R> f1 = cmk<R>((R)prm.e.f1re, (R)prm.e.f1im), f2 = cmk<R>((R)prm.e.f2re, (R)prm.e.f2im);
-#pragma unroll
-            for (int k = 0; k < 12; ++k) {
-                const Cplx<R> m = cmul(k < 6 ? f1 : f2, xv[k]);
-                Cplx<R> r       = cmk<R>(m.re - sc * acc[k].re, m.im - sc * acc[k].im);
-                if (prm.e.gamma5 && k >= 6) r = cmk<R>(-r.re, -r.im);
-                acc[k] = r;
-            }
-        }
-        SpinorIO<P>::store(prm.out, g.stride, i, acc);
-
-        if (DOT == DOT_Y) {
-            Cplx<R> yv[12];
-            SpinorIO<P>::load(prm.y, g.stride, i, yv);
-#pragma unroll
-            for (int k = 0; k < 12; ++k) {
-                const Cplx<R> p = cmulc(yv[k], acc[k]);
-                dv[0] += (double)p.re;
-                dv[1] += (double)p.im;
-            }
-        } else if (DOT == DOT_SELF) {
-#pragma unroll
-            for (int k = 0; k < 12; ++k) dv[0] += (double)acc[k].re * acc[k].re + (double)acc[k].im * acc[k].im;
-        }
-    }
-    if (DOT != DOT_NONE) {
-        __shared__ double smem[2 * 32];
-        block_sum<2>(dv, smem);
-        finish_reduction<2>(dv, prm.red, smem);
-    }
-}
 
 }  // namespace c2q

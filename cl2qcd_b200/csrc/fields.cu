@@ -8,7 +8,7 @@
 
 #include "blas_pk.cuh"
 #include "c2q_host.h"
-#include "dslash.cuh"
+#include "dslash64.cuh"
 
 namespace c2q {
 
@@ -98,6 +98,14 @@ HopCoef hop_coef(const c2q_gauge* g, double kappa)
     HopCoef c = g->coef;
     c.scale   = -kappa;
     return c;
+}
+
+bool adjoint_weights(const c2q_gauge* g)
+{
+    const HopCoef& c = g->coef;
+    for (int mu = 0; mu < 4; ++mu)
+        if (c.re[mu][0] != c.re[mu][1] || c.im[mu][0] != -c.im[mu][1]) return false;
+    return true;
 }
 
 // Site-diagonal factors (ocl_kernel/fermionmatrix_eo_m.cl:22-109, _m_merged.cl:22-64):
@@ -435,76 +443,77 @@ int gauge_drop_derived(c2q_gauge* g)
 }
 
 // ------------------------------------------------------------------ launches
-template <int P, int NL, int EPI, int DOT, int PH>
-static void dslash_go(const DslashParams<P>& prm, int blocks, cudaStream_t s)
+template <int NL, int EPI, int DOT>
+static void dslash_go(const Dslash64Params& prm, int blocks, cudaStream_t s)
 {
-    launch_dep(prm.pdl != 0, dslash_kernel<P, NL, EPI, DOT, PH>, dim3(blocks), dim3(128), 0, s, prm);
+    launch_dep(prm.pdl != 0, dslash64_kernel<NL, EPI, DOT>, dim3(blocks), dim3(128), 0, s, prm);
 }
 
-template <int P, int NL, int PH>
-static void dslash_dispatch_ph(const DslashParams<P>& prm, int epi, int dot, int blocks, cudaStream_t s)
+// (epilogue, reduction): 3 x 3 combinations, the CG residual update and <out, x>
+// with |out|^2 after EPI_AXPY, the CG solution update after EPI_PLAIN / EPI_DIAG
+template <int NL>
+static void dslash_dispatch(const Dslash64Params& prm, int epi, int dot, int blocks, cudaStream_t s)
 {
-    switch (epi * 3 + dot) {
-        case 0: dslash_go<P, NL, EPI_PLAIN, DOT_NONE, PH>(prm, blocks, s); break;
-        case 1: dslash_go<P, NL, EPI_PLAIN, DOT_Y, PH>(prm, blocks, s); break;
-        case 2: dslash_go<P, NL, EPI_PLAIN, DOT_SELF, PH>(prm, blocks, s); break;
-        case 3: dslash_go<P, NL, EPI_DIAG, DOT_NONE, PH>(prm, blocks, s); break;
-        case 4: dslash_go<P, NL, EPI_DIAG, DOT_Y, PH>(prm, blocks, s); break;
-        case 5: dslash_go<P, NL, EPI_DIAG, DOT_SELF, PH>(prm, blocks, s); break;
-        case 6: dslash_go<P, NL, EPI_AXPY, DOT_NONE, PH>(prm, blocks, s); break;
-        case 7: dslash_go<P, NL, EPI_AXPY, DOT_Y, PH>(prm, blocks, s); break;
-        case 8: dslash_go<P, NL, EPI_AXPY, DOT_SELF, PH>(prm, blocks, s); break;
+    switch (dot == DOT_CGR ? 9 : dot == DOT_OX ? 12 : dot == DOT_XUPD ? 10 + epi : epi * 3 + dot) {
+        case 0: dslash_go<NL, EPI_PLAIN, DOT_NONE>(prm, blocks, s); break;
+        case 1: dslash_go<NL, EPI_PLAIN, DOT_Y>(prm, blocks, s); break;
+        case 2: dslash_go<NL, EPI_PLAIN, DOT_SELF>(prm, blocks, s); break;
+        case 3: dslash_go<NL, EPI_DIAG, DOT_NONE>(prm, blocks, s); break;
+        case 4: dslash_go<NL, EPI_DIAG, DOT_Y>(prm, blocks, s); break;
+        case 5: dslash_go<NL, EPI_DIAG, DOT_SELF>(prm, blocks, s); break;
+        case 6: dslash_go<NL, EPI_AXPY, DOT_NONE>(prm, blocks, s); break;
+        case 7: dslash_go<NL, EPI_AXPY, DOT_Y>(prm, blocks, s); break;
+        case 8: dslash_go<NL, EPI_AXPY, DOT_SELF>(prm, blocks, s); break;
+        case 9: dslash_go<NL, EPI_AXPY, DOT_CGR>(prm, blocks, s); break;
+        case 10: dslash_go<NL, EPI_PLAIN, DOT_XUPD>(prm, blocks, s); break;
+        case 11: dslash_go<NL, EPI_DIAG, DOT_XUPD>(prm, blocks, s); break;
+        case 12: dslash_go<NL, EPI_AXPY, DOT_OX>(prm, blocks, s); break;
     }
 }
 
-// FP64 (bandwidth-bound) decides the phase pattern per launch.
-template <int P, int NL>
-static void dslash_dispatch(const DslashParams<P>& prm, int epi, int dot, int blocks, cudaStream_t s)
+static int dslash_fp64(c2q_ctx* ctx, const c2q_gauge* g, int gkind, c2q_spinor_eo* out, const c2q_spinor_eo* in,
+                       int out_parity, double kappa, int epi, const EpiArgs& e, const c2q_spinor_eo* x,
+                       const DotSpec& dot)
 {
-    dslash_dispatch_ph<P, NL, PH_ANY>(prm, epi, dot, blocks, s);
-}
-
-template <int P>
-static int dslash_typed(c2q_ctx* ctx, const c2q_gauge* g, int gkind, c2q_spinor_eo* out, const c2q_spinor_eo* in,
-                        int out_parity, double kappa, int epi, const EpiArgs& e, const c2q_spinor_eo* x,
-                        const DotSpec& dot)
-{
-    DslashParams<P> prm;
-    prm.out        = sptr<P>(out);
-    prm.in         = sptr<P>(in);
-    prm.x          = sptr<P>(x);
-    prm.y          = sptr<P>(dot.y);
+    Dslash64Params prm;
+    prm.out        = sptr<64>(out);
+    prm.in         = sptr<64>(in);
+    prm.x          = sptr<64>(x);
+    prm.y          = sptr<64>(dot.y);
     prm.gauge      = g->store[gkind].data;
     prm.g          = out->geom;
     prm.c          = hop_coef(g, kappa);
     prm.e          = e;
     prm.out_parity = out_parity;
     const int blocks = (out->geom.seo + 127) / 128;
-    if (dot.mode) {
-        int rc = ensure_partials(ctx, blocks);
+    const bool cgr = dot.mode == DOT_CGR, xup = dot.mode == DOT_XUPD;
+    if (dot.mode && !xup) {  // (DOT_OX reduces four doubles per block)
+        int rc = ensure_partials(ctx, dot.mode == DOT_OX ? 2 * (size_t)blocks : (size_t)blocks);
         if (rc) return rc;
     }
     prm.red = red_args(ctx, dot.fin);
     prm.pdl = ctx->pdl;
-    const bool r12 = gkind == G64R12 || gkind == G32R12 || gkind == G16R12;  // FP64 here
+    const bool r12 = gkind == G64R12;
     c2q_ctx::Timed tm{};
     if (ctx->profiling) {
         tm.a     = profile_event(ctx);
         tm.b     = profile_event(ctx);
-        tm.prec  = P;
+        tm.prec  = 64;
         tm.sites = (double)out->geom.seo;
         // compulsory traffic per output site: 8 links (each read once per sweep),
         // the input spinor (each read once through L2 reuse), the output, plus
-        // the epilogue/reduction operands read at the output site
+        // the epilogue/reduction operands read at the output site (a fused residual update reads and writes
+        // r and stores no output, a fused solution update reads p and reads and writes x)
         const double sp = 192.0;
         const double lk = (r12 ? 12.0 : 18.0) * 8.0;
-        tm.bytes = tm.sites * (8.0 * lk + sp * (2.0 + (epi == EPI_AXPY ? 1.0 : 0.0) + (dot.mode == DOT_Y ? 1.0 : 0.0)));
+        tm.bytes = tm.sites * (8.0 * lk + sp * (2.0 + (epi == EPI_AXPY ? 1.0 : 0.0) + (dot.mode == DOT_Y ? 1.0 : 0.0) +
+                                               (cgr ? 1.0 : 0.0) + (xup ? 3.0 : 0.0)));
         cudaEventRecord(tm.a, ctx->stream);
     }
     if (r12)
-        dslash_dispatch<P, 6>(prm, epi, dot.mode, blocks, ctx->stream);
+        dslash_dispatch<6>(prm, epi, dot.mode, blocks, ctx->stream);
     else
-        dslash_dispatch<P, 9>(prm, epi, dot.mode, blocks, ctx->stream);
+        dslash_dispatch<9>(prm, epi, dot.mode, blocks, ctx->stream);
     if (ctx->profiling) {
         cudaEventRecord(tm.b, ctx->stream);
         ctx->timed.push_back(tm);
@@ -534,7 +543,14 @@ int launch_dslash(c2q_ctx* ctx, const c2q_gauge* g, int gkind, c2q_spinor_eo* ou
     if (!gauge_matches(out->prec, gkind)) return fail(ctx, C2Q_BAD_ARG, "gauge precision mismatch");
     int rc = gauge_ensure(const_cast<c2q_gauge*>(g), gkind);
     if (rc) return rc;
-    if (out->prec == 64) return dslash_typed<64>(ctx, g, gkind, out, in, out_parity, kappa, epi, e, x, dot);
+    if (out->prec == 64) {
+        if (dot.mode == DOT_CGR || dot.mode == DOT_XUPD || dot.mode == DOT_OX) {
+            if ((dot.mode == DOT_XUPD) == (epi == EPI_AXPY) || !x || (dot.mode != DOT_OX && !dot.y))
+                return fail(ctx, C2Q_BAD_ARG, "fused update or reduction: wrong epilogue or missing operand");
+        }
+        return dslash_fp64(ctx, g, gkind, out, in, out_parity, kappa, epi, e, x, dot);
+    }
+    if (dot.mode == DOT_OX) return fail(ctx, C2Q_BAD_ARG, "the reduction with the operand is FP64");
     PkBatch B;
     B.n          = 1;
     B.out[0]     = out;
@@ -566,7 +582,8 @@ static int blas_typed(c2q_ctx* ctx, const BlasSpec& s, const c2q_spinor_eo* ref)
     A.stride = ref->geom.stride;
     A.op     = s.op;
     A.dot    = s.dot;
-    const int blocks = (A.n + BLAS_THREADS - 1) / BLAS_THREADS;
+    const int blocks = P == 64 ? (A.n + BLAS_THREADS - 1) / BLAS_THREADS
+                               : (A.n / 2 + BLAS_PK_THREADS - 1) / BLAS_PK_THREADS;
     if (s.dot) {  // dot 3 and 4 reduce four doubles per block
         int rc = ensure_partials(ctx, s.dot >= 3 ? 2 * (size_t)blocks : (size_t)blocks);
         if (rc) return rc;
@@ -610,8 +627,7 @@ static int cg_update_typed(c2q_ctx* ctx, c2q_spinor_eo* x, c2q_spinor_eo* r, con
     A.sc = ctx->scalars;
     A.n = x->geom.seo;
     A.stride = x->geom.stride;
-    const int blocks = P == 64 ? (A.n + BLAS_THREADS - 1) / BLAS_THREADS
-                               : (A.n / 2 + BLAS_PK_THREADS - 1) / BLAS_PK_THREADS;
+    const int blocks = (A.n + BLAS_THREADS - 1) / BLAS_THREADS;
     int rc = ensure_partials(ctx, blocks);
     if (rc) return rc;
     A.red = red_args(ctx, FIN_CG_BETA);
@@ -705,6 +721,33 @@ static int aee_sweeps(c2q_ctx* ctx, c2q_spinor_eo* out, const c2q_gauge* g, int 
     if (rc) return rc;
     EpiArgs e2 = tm ? diag_epi(mubar, minus ? C2Q_DIAG_M_TM_MINUS : C2Q_DIAG_M_TM, g5) : EpiArgs{1, 0, 1, 0, g5};
     return launch_dslash(ctx, g, gkind, out, tmp, /*EVEN -> odd sites*/ 1, kappa, EPI_AXPY, e2, in, dot);
+}
+
+int apply_qpqm_cg(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const c2q_spinor_eo* in, double kappa, double mubar,
+                  int action, c2q_spinor_eo* tmp1, c2q_spinor_eo* tmp2, c2q_spinor_eo* x, c2q_spinor_eo* r,
+                  int* sweeps)
+{
+    if (action != C2Q_ACTION_WILSON && action != C2Q_ACTION_TWISTEDMASS)
+        return fail(ctx, C2Q_BAD_ARG, "unknown fermion action (wilson or twistedmass)");
+    const bool tm = action == C2Q_ACTION_TWISTEDMASS;
+    DotSpec self, upx, upr;
+    self.mode = DOT_SELF;
+    self.fin  = FIN_CG_ALPHA;
+    upx.mode  = DOT_XUPD;
+    upx.y     = x;
+    upr.mode  = DOT_CGR;
+    upr.y     = r;
+    upr.fin   = FIN_CG_BETA;
+    int rc    = aee_sweeps(ctx, tmp2, g, gkind, in, kappa, mubar, action, 1, 1, tmp1, self);
+    if (!rc)
+        rc = launch_dslash(ctx, g, gkind, tmp1, tmp2, /*ODD -> even sites*/ 0, kappa, tm ? EPI_DIAG : EPI_PLAIN,
+                           tm ? diag_epi(mubar, C2Q_DIAG_M_TM_INVERSE, 0) : EpiArgs{1, 0, 1, 0, 0}, in, upx);
+    // (the last sweep stores no output: tmp2 stands in for the field it would write)
+    if (!rc)
+        rc = launch_dslash(ctx, g, gkind, tmp2, tmp1, /*EVEN -> odd sites*/ 1, kappa, EPI_AXPY,
+                           tm ? diag_epi(mubar, C2Q_DIAG_M_TM, 1) : EpiArgs{1, 0, 1, 0, 1}, tmp2, upr);
+    if (sweeps) *sweeps += 4;
+    return rc;
 }
 
 int apply_operator(c2q_ctx* ctx, int op, c2q_spinor_eo* out, const c2q_gauge* g, int gkind,

@@ -318,12 +318,7 @@ bool pcg64_applies(const c2q_ctx* ctx, int op, const c2q_gauge* gf)
 {
     // (per-launch timing wants the sweeps as launches of their own)
     if (op != C2Q_OP_QPLUSQMINUS_EO || ctx->profiling || gf->geom.seo > PCG64_MAX_SITES) return false;
-    // Q+ is the adjoint of Q- only where every backward weight is the conjugate of
-    // the forward one (no real chemical potential)
-    const HopCoef& c = gf->coef;
-    for (int mu = 0; mu < 4; ++mu)
-        if (c.re[mu][0] != c.re[mu][1] || c.im[mu][0] != -c.im[mu][1]) return false;
-    return true;
+    return adjoint_weights(gf);
 }
 
 int pcg64_run(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const Pcg64Solve& S, Pcg64Result* out)

@@ -10,6 +10,7 @@
 
 #include "blas.cuh"
 #include "c2q_host.h"
+#include "dslash64.cuh"
 #include "mixed.cuh"
 
 namespace c2q {
@@ -239,6 +240,25 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
     const int gk = gk64_for(g, P->use_rec12);
     int sweeps   = 0;
     SolveClock clock(ctx);
+    const bool small = pcg64_applies(ctx, op, g);
+    // Q+Q- with the vector updates in its sweeps
+    const bool fused = !small && op == C2Q_OP_QPLUSQMINUS_EO && adjoint_weights(g);
+    // rn = b - A x, omega = |rn|^2, p = rn
+    auto refresh = [&]() -> int {
+        int e = apply_operator(ctx, op, rn, g, gk, x, kappa, mubar, action, t1, t2, DotSpec{}, &sweeps);
+        if (!e) e = saxpy_norm(ctx, rn, Cx{1, 0}, rn, b, FIN_CG_OMEGA, nullptr);
+        return e ? e : copy_field(ctx, p, rn);
+    };
+    // v = A p with (p, v) -> alpha; x += alpha p; rn -= alpha v; beta, omega
+    auto apply_update = [&](int* sw) -> int {
+        if (fused) return apply_qpqm_cg(ctx, g, gk, p, kappa, mubar, action, t1, t2, x, rn, sw);
+        DotSpec d;
+        d.mode = DOT_Y;
+        d.y    = p;
+        d.fin  = FIN_CG_ALPHA;
+        int e  = apply_operator(ctx, op, v, g, gk, p, kappa, mubar, action, t1, t2, d, sw);
+        return e ? e : launch_cg_update(ctx, x, rn, p, v);
+    };
 
     double b2 = 0;
     rc        = saxpy_norm(ctx, rn, Cx{0, 0}, b, b, FIN_STORE_RESULT, &b2);
@@ -252,7 +272,7 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
     double resid = std::numeric_limits<double>::quiet_NaN();
     bool force_refresh = false;
     double r2_confirmed = -1.0;  // true residual of the returned solution, when already computed
-    if (pcg64_applies(ctx, op, g)) {
+    if (small) {
         // Small lattices: everything between two refreshes in one launch.  With
         // rel_tol every residual is judged, one iteration after its own as below,
         // and a converged one confirmed by a true residual; else every
@@ -264,9 +284,7 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
             Pcg64Solve S{x, rn, p, t1, t2, kappa, mubar, action};
             if (iter % P->iter_refresh == 0 || force_refresh) {
                 force_refresh = false;
-                rc = apply_operator(ctx, op, rn, g, gk, x, kappa, mubar, action, t1, t2, DotSpec{}, &sweeps);
-                if (!rc) rc = saxpy_norm(ctx, rn, Cx{1, 0}, rn, b, FIN_CG_OMEGA, nullptr);
-                if (!rc) rc = copy_field(ctx, p, rn);
+                rc            = refresh();
                 if (rc) return rc;
                 S.p_ready = 1;
             }
@@ -325,20 +343,10 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
         } gexec;
         long long gkernels = 0;
         int gsweeps        = 0;
-        auto apply_update = [&](int* sw) -> int {
-            DotSpec d;
-            d.mode = DOT_Y;
-            d.y    = p;
-            d.fin  = FIN_CG_ALPHA;
-            int e  = apply_operator(ctx, op, v, g, gk, p, kappa, mubar, action, t1, t2, d, sw);
-            return e ? e : launch_cg_update(ctx, x, rn, p, v);
-        };
         for (iter = 0; iter < P->cgmax || iter < P->min_iter; iter++) {
             if (iter % P->iter_refresh == 0 || force_refresh) {
                 force_refresh = false;
-                rc = apply_operator(ctx, op, rn, g, gk, x, kappa, mubar, action, t1, t2, DotSpec{}, &sweeps);
-                if (!rc) rc = saxpy_norm(ctx, rn, Cx{1, 0}, rn, b, FIN_CG_OMEGA, nullptr);
-                if (!rc) rc = copy_field(ctx, p, rn);
+                rc            = refresh();
                 if (!rc) rc = apply_update(&sweeps);
             } else if (graphs) {
                 if (!gexec.e) {
@@ -396,17 +404,10 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
         for (iter = 0; iter < P->cgmax || iter < P->min_iter; iter++) {
             if (iter % P->iter_refresh == 0 || force_refresh) {
                 force_refresh = false;
-                rc = apply_operator(ctx, op, rn, g, gk, x, kappa, mubar, action, t1, t2, DotSpec{}, &sweeps);
-                if (!rc) rc = saxpy_norm(ctx, rn, Cx{1, 0}, rn, b, FIN_CG_OMEGA, nullptr);  // rn = b - A x ; omega = (rn,rn)
-                if (!rc) rc = copy_field(ctx, p, rn);
+                rc            = refresh();
                 if (rc) return rc;
             }
-            DotSpec d;
-            d.mode = DOT_Y;
-            d.y    = p;
-            d.fin  = FIN_CG_ALPHA;  // rho = (p, v) ; alpha = omega / rho
-            rc     = apply_operator(ctx, op, v, g, gk, p, kappa, mubar, action, t1, t2, d, &sweeps);
-            if (!rc) rc = launch_cg_update(ctx, x, rn, p, v);  // x += alpha p ; rn -= alpha v ; beta, omega
+            rc = apply_update(&sweeps);
             if (rc) return rc;
             if (iter % P->resid_check_every == 0) {
                 SolverScalars h;
@@ -1243,6 +1244,18 @@ struct BicgLoop {
     {
         return blas(B_SAXPY, nullptr, none, X, none, Y, nullptr, kind, fin, fin_arg);
     }
+    // t = A s; (t, s), (t, t): omega -- reduced in the last sweep where s is its operand
+    int apply_ts()
+    {
+        if (sp.prec == 64 && A == 2) {
+            DotSpec d;
+            d.mode = DOT_OX;
+            d.fin  = FIN_BI_OMEGA;
+            return sp.apply_dot(t, s, d);
+        }
+        const int e = sp.apply(t, s);
+        return e ? e : dot(t, s, 3, FIN_BI_OMEGA);
+    }
     // bicgstab.cpp:612-723 (the x update, the rn update and the two reductions
     // that follow them run as one pass, B_BICG_XR).  refresh 2: x is zero, so
     // rn = b without applying the operator.
@@ -1262,8 +1275,7 @@ struct BicgLoop {
         }
         if (!e) e = sp.apply_dot(v, p, alpha_dot);  // v = A p; tmp1 = (rhat, v); alpha
         if (!e) e = blas(B_SAXPY, s, coef_dev(sc->alpha), v, none, rn, nullptr);  // s = rn - alpha v
-        if (!e) e = sp.apply(t, s);
-        if (!e) e = dot(t, s, 3, FIN_BI_OMEGA);
+        if (!e) e = apply_ts();
         if (!e) {  // x += alpha p + omega s; rn = s - omega t; |rn|^2, (rhat, rn): beta and the tests
             BlasSpec q;
             q.op      = B_BICG_XR;
@@ -1298,8 +1310,7 @@ struct BicgLoop {
         if (!e) e = blas(B_SAXSBYPZ, p, coef_dev(sc->beta), p, coef_dev(sc->tmp2), v, rn);
         if (!e) e = sp.apply_dot(v, p, alpha_dot);
         if (!e) e = blas(B_SAXPY, s, coef_dev(sc->alpha), v, none, rn, nullptr);
-        if (!e) e = sp.apply(t, s);
-        if (!e) e = dot(t, s, 3, FIN_BI_OMEGA);
+        if (!e) e = apply_ts();
         if (!e) e = blas(B_SAXSBYPZ, x, coef_dev(sc->alpha), p, coef_dev(sc->omega), s, x);
         if (!e) e = blas(B_SAXPY, rn, coef_dev(sc->omega), t, none, s, nullptr, 2, FIN_BI_RESID, 1);
         return e;
@@ -1356,13 +1367,17 @@ int bicgstab_dev(EoSpace& sp, c2q_spinor_eo* x, c2q_spinor_eo* b, const c2q_solv
     auto save_iter = [&](int, bool refresh) { return L.save_iter(x, b, refresh); };
     auto push      = [&](int k) { return L.push(k); };
     auto pop       = [&](int k, double* r, int* h) { return L.pop(k, r, h); };
+    // |b - A x|^2 into *tr
+    auto true_r2 = [&](double* tr) -> int {
+        int e = sp.apply(aux, x);
+        if (!e) e = blas(B_SAXPY, aux, one, aux, none, b, nullptr, 2, FIN_STORE_RESULT);
+        return e ? e : read_scalars(ctx, ctx->red_result, 2, tr);
+    };
     // the true-residual confirmation (save variant, rel_tol); unpredicated
     auto confirmed = [&](bool* ok) -> int {
         ctx->halt_dev = nullptr;
-        int e         = sp.apply(aux, x);
-        if (!e) e = blas(B_SAXPY, aux, one, aux, none, b, nullptr, 2, FIN_STORE_RESULT);
-        double tr[2] = {0, 0};
-        if (!e) e = read_scalars(ctx, ctx->red_result, 2, tr);
+        double tr[2]  = {0, 0};
+        const int e   = true_r2(tr);
         ctx->halt_dev = &sc->halt;
         const double lim = P->rel_tol > 0 ? std::max(P->rel_tol * P->rel_tol * b2, P->prec > 0 ? P->prec : 0.0)
                                           : P->prec;
@@ -1465,10 +1480,8 @@ int bicgstab_dev(EoSpace& sp, c2q_spinor_eo* x, c2q_spinor_eo* b, const c2q_solv
     ctx->halt_dev = nullptr;
     double r2t    = 0;
     {
-        rc = sp.apply(aux, x);
-        if (!rc) rc = blas(B_SAXPY, aux, one, aux, none, b, nullptr, 2, FIN_STORE_RESULT);
         double tr[2] = {0, 0};
-        if (!rc) rc = read_scalars(ctx, ctx->red_result, 2, tr);
+        rc           = true_r2(tr);
         if (rc) return rc;
         r2t = tr[0];
         executed += A;
