@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <map>
 #include <string>
 #include <vector>
@@ -165,6 +166,14 @@ int gkind_for(int prec, int rec12);
 int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f, bool clear = false);
 void field_free(c2q_spinor_eo* f);
 size_t field_bytes(const Geom& g, int prec);
+// Memory of the gauge objects (links, derived copies, momenta) from the same pool as
+// the spinor fields, in stream order: a program that replaces a gauge field gets
+// the freed blocks back instead of new mappings (some milliseconds of the first solve
+// on a new field).  link_free waits for the device, as other contexts may still read the
+// block, and gives back what the pool holds unused beyond POOL_KEEP.
+constexpr size_t POOL_KEEP = (size_t)22 << 30;  // an eighth of a B200
+cudaError_t link_alloc(c2q_ctx* ctx, void** p, size_t bytes);
+void link_free(c2q_ctx* ctx, std::initializer_list<void*> blocks);
 int gauge_ensure(c2q_gauge* g, int kind);  // builds a lower-precision copy on first use
 // frees every copy derived from the FP64 18-real links (rebuilt on next use)
 int gauge_drop_derived(c2q_gauge* g);

@@ -366,6 +366,27 @@ __global__ void gauge_convert16_kernel(const double2* __restrict__ in, uint4* __
     }
 }
 
+cudaError_t link_alloc(c2q_ctx* ctx, void** p, size_t bytes)
+{
+    const cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
+void link_free(c2q_ctx* ctx, std::initializer_list<void*> blocks)
+{
+    cudaDeviceSynchronize();
+    for (void* p : blocks)
+        if (p) cudaFreeAsync(p, ctx->stream);
+    cudaMemPool_t pool;
+    uint64_t held = 0, used = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) != cudaSuccess) return;
+    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) return;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return;
+    if (held > used + POOL_KEEP) cudaMemPoolTrimTo(pool, used + POOL_KEEP);
+}
+
 int gauge_ensure(c2q_gauge* g, int kind)
 {
     c2q_ctx* ctx = g->ctx;
@@ -387,18 +408,18 @@ int gauge_ensure(c2q_gauge* g, int kind)
     const double2* src = static_cast<const double2*>(g->store[G64].data);
     void* tmp          = nullptr;  // temporal gauge: the transformed FP64 links
     if (gkind_is_tg(kind)) {
-        C2Q_CUDA(ctx, cudaMalloc(&tmp, lanes * 9 * 16));
+        C2Q_CUDA(ctx, link_alloc(ctx, &tmp, lanes * 9 * 16));
         const int rc = tg_links_fp64(g, tmp);
         if (rc) {
-            cudaFree(tmp);
+            cudaFreeAsync(tmp, ctx->stream);
             return rc;
         }
         src = static_cast<const double2*>(tmp);
     }
     void* p = nullptr;
-    const cudaError_t ea = cudaMalloc(&p, bytes);
+    const cudaError_t ea = link_alloc(ctx, &p, bytes);
     if (ea != cudaSuccess) {
-        cudaFree(tmp);
+        if (tmp) cudaFreeAsync(tmp, ctx->stream);
         return cuda_fail(ctx, ea, "cudaMalloc(gauge copy)");
     }
     const int threads = 256;
@@ -416,12 +437,11 @@ int gauge_ensure(c2q_gauge* g, int kind)
     }
     ctx->launches++;
     const cudaError_t ek = cudaGetLastError();
-    if (tmp) {  // stream-ordered: the conversion finishes before the scratch is released
-        cudaStreamSynchronize(ctx->stream);
-        cudaFree(tmp);
-    }
+    if (tmp) cudaFreeAsync(tmp, ctx->stream);
+    // (the copy may be read on other streams)
+    cudaStreamSynchronize(ctx->stream);
     if (ek != cudaSuccess) {
-        cudaFree(p);
+        cudaFreeAsync(p, ctx->stream);
         return cuda_fail(ctx, ek, "gauge conversion");
     }
     g->store[kind].data  = p;
@@ -432,12 +452,14 @@ int gauge_ensure(c2q_gauge* g, int kind)
 int gauge_drop_derived(c2q_gauge* g)
 {
     c2q_ctx* ctx = g->ctx;
+    bool any = g->tg_transform.data != nullptr;
+    for (int k = 1; k < GAUGE_KINDS; ++k) any = any || g->store[k].data;
     C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    for (int k = 1; k < GAUGE_KINDS; ++k) {
-        cudaFree(g->store[k].data);
-        g->store[k] = GaugeStore{};
-    }
-    cudaFree(g->tg_transform.data);
+    if (!any) return C2Q_OK;
+    link_free(ctx, {g->store[1].data, g->store[2].data, g->store[3].data, g->store[4].data, g->store[5].data,
+                    g->store[6].data, g->store[7].data, g->store[8].data, g->store[9].data, g->tg_transform.data});
+    static_assert(GAUGE_KINDS == 10, "every derived copy is freed above");
+    for (int k = 1; k < GAUGE_KINDS; ++k) g->store[k] = GaugeStore{};
     g->tg_transform = GaugeStore{};
     return C2Q_OK;
 }
@@ -937,7 +959,7 @@ C2Q_EXPORT int c2q_gauge_create(c2q_ctx* ctx, const c2q_lattice* lat, c2q_gauge*
     }
     g->coef            = hop_coef(*lat, 0.0);
     const size_t bytes = (size_t)8 * 9 * g->geom.stride * 16;
-    cudaError_t e      = cudaMalloc(&g->store[G64].data, bytes);
+    cudaError_t e      = link_alloc(ctx, &g->store[G64].data, bytes);
     if (e != cudaSuccess) {
         delete g;
         return cuda_fail(ctx, e, "cudaMalloc(gauge)");
@@ -951,9 +973,8 @@ C2Q_EXPORT int c2q_gauge_create(c2q_ctx* ctx, const c2q_lattice* lat, c2q_gauge*
 C2Q_EXPORT int c2q_gauge_destroy(c2q_gauge* g)
 {
     if (!g) return C2Q_OK;
-    cudaStreamSynchronize(g->ctx->stream);
-    for (auto& s : g->store) cudaFree(s.data);
-    cudaFree(g->tg_transform.data);
+    gauge_drop_derived(g);
+    link_free(g->ctx, {g->store[G64].data});
     delete g;
     return C2Q_OK;
 }

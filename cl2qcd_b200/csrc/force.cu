@@ -236,13 +236,13 @@ C2Q_EXPORT int c2q_gaugemomenta_create(c2q_ctx* ctx, const c2q_lattice* lat, c2q
     m->lat   = *lat;
     m->geom  = g;
     m->bytes = (size_t)2 * 4 * 8 * g.stride * sizeof(double);
-    if (cudaMalloc(&m->data, m->bytes) != cudaSuccess) {
+    if (link_alloc(ctx, reinterpret_cast<void**>(&m->data), m->bytes) != cudaSuccess) {
         delete m;
         return fail(ctx, C2Q_OOM, "gauge momenta: out of device memory");
     }
     const cudaError_t e = cudaMemsetAsync(m->data, 0, m->bytes, ctx->stream);
     if (e != cudaSuccess) {
-        cudaFree(m->data);
+        cudaFreeAsync(m->data, ctx->stream);
         delete m;
         return cuda_fail(ctx, e, "cudaMemsetAsync(gauge momenta)");
     }
@@ -253,8 +253,7 @@ C2Q_EXPORT int c2q_gaugemomenta_create(c2q_ctx* ctx, const c2q_lattice* lat, c2q
 C2Q_EXPORT int c2q_gaugemomenta_destroy(c2q_gaugemomenta* m)
 {
     if (!m) return C2Q_OK;
-    cudaStreamSynchronize(m->ctx->stream);
-    cudaFree(m->data);
+    link_free(m->ctx, {m->data});
     delete m;
     return C2Q_OK;
 }

@@ -229,7 +229,7 @@ int tg_ensure(c2q_gauge* g)
     }
     const size_t bytes = (size_t)2 * 9 * g->geom.stride * sizeof(double2);
     void* p            = nullptr;
-    C2Q_CUDA(ctx, cudaMalloc(&p, bytes));
+    C2Q_CUDA(ctx, link_alloc(ctx, &p, bytes));
     C2Q_CUDA(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));
     const int vs = g->lat.ns * g->lat.ns * g->lat.ns;
     tg_transform_kernel<<<(vs + 127) / 128, 128, 0, ctx->stream>>>(static_cast<const double2*>(g->store[G64].data),
@@ -237,7 +237,7 @@ int tg_ensure(c2q_gauge* g)
     ctx->launches++;
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
-        cudaFree(p);
+        cudaFreeAsync(p, ctx->stream);
         return cuda_fail(ctx, e, "tg_transform_kernel");
     }
     g->tg_transform.data  = p;
