@@ -319,7 +319,9 @@ struct PcgResult {
 // 20^3x40 (625 tiles) 110 against 104, four sources at 16^3x32 165 against 144.
 int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* most);
 size_t pcg_ctl_bytes();
-int pcg_run(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B, PcgResult* out);
+// launch without waiting; collect waits for the stream, and so for what was queued since
+int pcg_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B);
+int pcg_collect(c2q_ctx* ctx, const PcgBatch& B, PcgResult* out);
 // Iterations of the FP64 CG on QplusQminus_eo in one cooperative launch
 // (pcg64.cu), with the context's solver scalars: until a judged residual is
 // below thr (from iteration min_iter on) or no number, or `iters` are done.

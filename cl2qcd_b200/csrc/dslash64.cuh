@@ -4,7 +4,7 @@
 // Bound by HBM: 8 links of 144 bytes, the neighbours through L2 and the output, 1536
 // bytes a site, at 94 % of the measured copy rate on 24^3x48.  The vector updates of the
 // CG and BiCGStab's (t, s) ride along where their operands are at hand (DOT_XUPD,
-// DOT_CGR, DOT_OX), each saving the passes of its own kernel over p, v, x and r.
+// DOT_CGR, DOT_OX, DOT_RES), each saving the passes of its own kernel over p, v, x and r.
 // (In the temporal gauge, with a fifth fewer bytes, the sweep was no faster: 97 us
 // against 83 us; prefetching the next direction's links to L2 did not change that.)
 #pragma once
@@ -16,6 +16,8 @@ namespace c2q {
 // <out, x> and |out|^2 with the EPI_AXPY operand x, from registers: BiCGStab's
 // (t, s) and (t, t) for t = A s.
 constexpr int DOT_OX = 5;
+// out = y - (EPI_AXPY result) with |out|^2: the true residual b - A x, y = b.
+constexpr int DOT_RES = 6;
 
 struct Dslash64Params {
     SpinorPtr<64> out;
@@ -133,6 +135,15 @@ __global__ void __launch_bounds__(128) dslash64_kernel(const Dslash64Params prm)
                     dv[2] += q.re;
                     dv[3] += q.im;
                 }
+            }
+        }
+        if (DOT == DOT_RES) {
+            C yv[12];
+            SpinorIO<64>::load(prm.y, g.stride, i, yv);
+#pragma unroll
+            for (int k = 0; k < 12; ++k) {
+                acc[k] = yv[k] - acc[k];
+                dv[0] += acc[k].re * acc[k].re + acc[k].im * acc[k].im;
             }
         }
         if (DOT != DOT_CGR) SpinorIO<64>::store(prm.out, g.stride, i, acc);

@@ -471,12 +471,12 @@ static void dslash_go(const Dslash64Params& prm, int blocks, cudaStream_t s)
     launch_dep(prm.pdl != 0, dslash64_kernel<NL, EPI, DOT>, dim3(blocks), dim3(128), 0, s, prm);
 }
 
-// (epilogue, reduction): 3 x 3 combinations, the CG residual update and <out, x>
-// with |out|^2 after EPI_AXPY, the CG solution update after EPI_PLAIN / EPI_DIAG
+// (epilogue, reduction): 3 x 3 combinations, the CG residual update, <out, x>
+// with |out|^2 and the true residual after EPI_AXPY, the CG solution update after EPI_PLAIN / EPI_DIAG
 template <int NL>
 static void dslash_dispatch(const Dslash64Params& prm, int epi, int dot, int blocks, cudaStream_t s)
 {
-    switch (dot == DOT_CGR ? 9 : dot == DOT_OX ? 12 : dot == DOT_XUPD ? 10 + epi : epi * 3 + dot) {
+    switch (dot == DOT_CGR ? 9 : dot == DOT_OX ? 12 : dot == DOT_RES ? 13 : dot == DOT_XUPD ? 10 + epi : epi * 3 + dot) {
         case 0: dslash_go<NL, EPI_PLAIN, DOT_NONE>(prm, blocks, s); break;
         case 1: dslash_go<NL, EPI_PLAIN, DOT_Y>(prm, blocks, s); break;
         case 2: dslash_go<NL, EPI_PLAIN, DOT_SELF>(prm, blocks, s); break;
@@ -490,6 +490,7 @@ static void dslash_dispatch(const Dslash64Params& prm, int epi, int dot, int blo
         case 10: dslash_go<NL, EPI_PLAIN, DOT_XUPD>(prm, blocks, s); break;
         case 11: dslash_go<NL, EPI_DIAG, DOT_XUPD>(prm, blocks, s); break;
         case 12: dslash_go<NL, EPI_AXPY, DOT_OX>(prm, blocks, s); break;
+        case 13: dslash_go<NL, EPI_AXPY, DOT_RES>(prm, blocks, s); break;
     }
 }
 
@@ -528,7 +529,7 @@ static int dslash_fp64(c2q_ctx* ctx, const c2q_gauge* g, int gkind, c2q_spinor_e
         // r and stores no output, a fused solution update reads p and reads and writes x)
         const double sp = 192.0;
         const double lk = (r12 ? 12.0 : 18.0) * 8.0;
-        tm.bytes = tm.sites * (8.0 * lk + sp * (2.0 + (epi == EPI_AXPY ? 1.0 : 0.0) + (dot.mode == DOT_Y ? 1.0 : 0.0) +
+        tm.bytes = tm.sites * (8.0 * lk + sp * (2.0 + (epi == EPI_AXPY ? 1.0 : 0.0) + (dot.mode == DOT_Y || dot.mode == DOT_RES ? 1.0 : 0.0) +
                                                (cgr ? 1.0 : 0.0) + (xup ? 3.0 : 0.0)));
         cudaEventRecord(tm.a, ctx->stream);
     }
@@ -566,13 +567,14 @@ int launch_dslash(c2q_ctx* ctx, const c2q_gauge* g, int gkind, c2q_spinor_eo* ou
     int rc = gauge_ensure(const_cast<c2q_gauge*>(g), gkind);
     if (rc) return rc;
     if (out->prec == 64) {
-        if (dot.mode == DOT_CGR || dot.mode == DOT_XUPD || dot.mode == DOT_OX) {
+        if (dot.mode == DOT_CGR || dot.mode == DOT_XUPD || dot.mode == DOT_OX || dot.mode == DOT_RES) {
             if ((dot.mode == DOT_XUPD) == (epi == EPI_AXPY) || !x || (dot.mode != DOT_OX && !dot.y))
                 return fail(ctx, C2Q_BAD_ARG, "fused update or reduction: wrong epilogue or missing operand");
         }
         return dslash_fp64(ctx, g, gkind, out, in, out_parity, kappa, epi, e, x, dot);
     }
-    if (dot.mode == DOT_OX) return fail(ctx, C2Q_BAD_ARG, "the reduction with the operand is FP64");
+    if (dot.mode == DOT_OX || dot.mode == DOT_RES)
+        return fail(ctx, C2Q_BAD_ARG, "this fused reduction is FP64");
     PkBatch B;
     B.n          = 1;
     B.out[0]     = out;

@@ -32,6 +32,9 @@ int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* most)
     return C2Q_OK;
 }
 
+// where the control block lands in the context's pinned buffer (read_scalars uses its head)
+constexpr int PCG_PINNED = 16;
+
 size_t pcg_ctl_bytes() { return sizeof(PcgCtl); }
 
 template <int P, int NL>
@@ -47,7 +50,7 @@ static int pcg_go(c2q_ctx* ctx, PcgParams& prm)
     return C2Q_OK;
 }
 
-int pcg_run(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B, PcgResult* out)
+int pcg_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B)
 {
     PcgParams prm;
     memset(&prm, 0, sizeof prm);
@@ -89,12 +92,15 @@ int pcg_run(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B, PcgR
     else
         rc = gkind_is_r12(gkind) ? pcg_go<32, 6>(ctx, prm) : pcg_go<32, 9>(ctx, prm);
     if (rc) return rc;
-    static_assert(sizeof(PcgCtl) <= 64 * sizeof(double), "the control block fits the context's pinned buffer");
-    rc = pinned_copy(ctx, ctx->host_pinned_dev, 0, prm.ctl, 0, sizeof(PcgCtl));
-    if (rc) return rc;
+    static_assert(sizeof(PcgCtl) <= (64 - PCG_PINNED) * sizeof(double), "the control block fits the pinned buffer");
+    return pinned_copy(ctx, ctx->host_pinned_dev + PCG_PINNED, 0, prm.ctl, 0, sizeof(PcgCtl));
+}
+
+int pcg_collect(c2q_ctx* ctx, const PcgBatch& B, PcgResult* out)
+{
     C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     PcgCtl c;
-    memcpy(&c, ctx->host_pinned, sizeof c);
+    memcpy(&c, ctx->host_pinned + PCG_PINNED, sizeof c);
     if (c.error || c.iters < 1) return fail(ctx, C2Q_CUDA_ERROR, "cooperative CG: a grid barrier gave up");
     out->iters = c.iters;
     for (int r = 0; r < B.n; ++r) {

@@ -143,9 +143,16 @@ int true_residual(c2q_ctx* ctx, int op, const c2q_gauge* g, const c2q_spinor_eo*
                   double kappa, double mubar, int action, c2q_spinor_eo* r, c2q_spinor_eo* t1, c2q_spinor_eo* t2,
                   double* r2, int* sweeps, int gk64 = G64)
 {
-    int rc = apply_operator(ctx, op, r, g, gk64, x, kappa, mubar, action, t1, t2, DotSpec{}, sweeps);
+    DotSpec d;  // the subtraction and the norm ride in the operator's last sweep
+    d.mode = DOT_RES;
+    d.y    = b;
+    d.fin  = FIN_STORE_RESULT;
+    int rc = apply_operator(ctx, op, r, g, gk64, x, kappa, mubar, action, t1, t2, d, sweeps);
     if (rc) return rc;
-    return saxpy_norm(ctx, r, Cx{1, 0}, r, b, FIN_STORE_RESULT, r2);
+    double h[2];
+    rc  = read_scalars(ctx, ctx->red_result, 2, h);
+    *r2 = h[0];
+    return rc;
 }
 
 // |x|^2 (to skip A x when the start vector is zero)
@@ -245,8 +252,11 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
     const bool fused = !small && op == C2Q_OP_QPLUSQMINUS_EO && adjoint_weights(g);
     // rn = b - A x, omega = |rn|^2, p = rn
     auto refresh = [&]() -> int {
-        int e = apply_operator(ctx, op, rn, g, gk, x, kappa, mubar, action, t1, t2, DotSpec{}, &sweeps);
-        if (!e) e = saxpy_norm(ctx, rn, Cx{1, 0}, rn, b, FIN_CG_OMEGA, nullptr);
+        DotSpec d;
+        d.mode = DOT_RES;
+        d.y    = b;
+        d.fin  = FIN_CG_OMEGA;
+        int e  = apply_operator(ctx, op, rn, g, gk, x, kappa, mubar, action, t1, t2, d, &sweeps);
         return e ? e : copy_field(ctx, p, rn);
     };
     // v = A p with (p, v) -> alpha; x += alpha p; rn -= alpha v; beta, omega
@@ -526,6 +536,12 @@ int accumulate(c2q_ctx* ctx, c2q_spinor_eo* x, c2q_spinor_eo* xs, const c2q_spin
     return C2Q_OK;
 }
 
+// A right-hand side's scalars at the start (zeroed before): omega = (r, r).
+__global__ void mixed_start_kernel(SolverScalars* s, double r2)
+{
+    if (threadIdx.x == 0) s->omega[0] = r2;
+}
+
 // A reliable update's scalars: beta rescaled to the true residual r2 (the
 // search direction is kept), omega = resid = r2, alpha = 0 (the deferred x
 // update was accumulated).
@@ -617,14 +633,6 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
     const double delta = P->reliable_delta > 0 ? P->reliable_delta : 0.1;
     SolveClock clock(ctx);
 
-    auto write_one = [&](int k, const SolverScalars& h) -> int {
-        memcpy(ctx->host_pinned, &h, sizeof(SolverScalars));
-        const int rc1 = pinned_copy(ctx, dsc + k, 0, ctx->host_pinned_dev, 0, sizeof(SolverScalars));
-        if (rc1) return rc1;
-        C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        return C2Q_OK;
-    };
-
     auto to_inner = [&](c2q_spinor_eo* out, const c2q_spinor_eo* in) -> int {
         return use_tg ? tg_to_inner(ctx, g, out, in) : launch_convert(ctx, out, in);
     };
@@ -659,10 +667,10 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
         }
         rc = c2q_spinor_eo_zero(xs[k]);
         if (!rc) rc = launch_convert(ctx, p[k], rs[k]);
-        SolverScalars h0{};
-        h0.omega[0] = s.r2;
-        if (!rc) rc = write_one(k, h0);
         if (rc) return rc;
+        mixed_start_kernel<<<1, 32, 0, ctx->stream>>>(dsc + k, s.r2);
+        ctx->launches++;
+        C2Q_CUDA(ctx, cudaGetLastError());
         s.maxrr  = std::sqrt(s.r2);
         s.active = true;
     }
@@ -735,6 +743,9 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
         if (act.empty()) break;
         hist[iter % 4]   = act;
         const bool whole = (int)act.size() <= whole_most;
+        bool spec        = false;  // the update's residual is there already (r2_spec, on links gk_spec)
+        int gk_spec      = G64;
+        double r2_spec   = 0;
         if (whole) {
             PcgBatch C;
             PcgResult R;
@@ -758,7 +769,21 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
             C.first  = iter == 0;
             C.iters  = P->cgmax - iter;
             C.ctl    = dsc + n;
-            rc       = pcg_run(ctx, g, gk, C, &R);
+            rc       = pcg_launch(ctx, g, gk, C);
+            // A right-hand side alone: whatever ended the iterations, its increment
+            // goes into x and the true residual is due, so both are queued behind them
+            // without asking.  The update that is expected to be the last takes the
+            // links as uploaded, as below: its residual has no room above thr.
+            const int k0 = act[0];
+            spec         = C.n == 1;
+            if (!rc && spec) {
+                gk_spec = delta * delta * S[k0].maxrr * S[k0].maxrr < S[k0].thr ? G64 : gk64;
+                rc      = take_out(k0, nullptr);
+                if (!rc)
+                    rc = true_residual(ctx, op, g, x[k0], b[k0], kappa, mubar, action, r64, a64, b64, &r2_spec,
+                                       &S[k0].sweeps, gk_spec);
+            }
+            if (!rc) rc = pcg_collect(ctx, C, &R);
             if (rc) return rc;
             iter += R.iters - 1;  // the last iteration done
             hist[(iter + 3) % 4] = act;
@@ -826,11 +851,15 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
                 // reliable update in FP64 after iteration `iter`
                 // (an update expected to be the last one uses the uploaded links;
                 // one that converges unexpectedly on 12-real links is confirmed on them)
-                rc = take_out(k, fused ? nullptr : dsc + k);
-                const int gk_upd = resid < s.thr ? G64 : gk64;
-                if (!rc)
-                    rc = true_residual(ctx, op, g, x[k], b[k], kappa, mubar, action, r64, a64, b64, &s.r2, &s.sweeps,
-                                       gk_upd);
+                const int gk_upd = spec ? gk_spec : resid < s.thr ? G64 : gk64;
+                if (spec) {
+                    s.r2 = r2_spec;
+                } else {
+                    rc = take_out(k, fused ? nullptr : dsc + k);
+                    if (!rc)
+                        rc = true_residual(ctx, op, g, x[k], b[k], kappa, mubar, action, r64, a64, b64, &s.r2,
+                                           &s.sweeps, gk_upd);
+                }
                 if (!rc && gk_upd != G64 && s.r2 < s.thr)
                     rc = true_residual(ctx, op, g, x[k], b[k], kappa, mubar, action, r64, a64, b64, &s.r2, &s.sweeps,
                                        G64);

@@ -19,6 +19,7 @@
 // (the gauge store layout without the direction).
 #include <cmath>
 
+#include "blas_pk.cuh"
 #include "c2q_host.h"
 
 namespace c2q {
@@ -143,60 +144,75 @@ __global__ void tg_links_kernel(const double2* __restrict__ U, const double2* __
     store9(out + (size_t)(par * 4 + mu) * 9 * g.stride, g.stride, i, r);
 }
 
-// out = G in on the parity-1 sites (the CG vectors), FP64 arithmetic
-template <int PO>
-__global__ void __launch_bounds__(BLAS_THREADS) tg_to_inner_kernel(SpinorPtr<PO> out, SpinorPtr<64> in,
-                                                                   const double2* __restrict__ G1, int n, int stride)
+// out = G in on the parity-1 sites (the CG vectors), FP64 arithmetic; FP32 out in
+// slots, one thread per slot (its sites j and j + n / 2): whole words of the slot layout
+__global__ void __launch_bounds__(128) tg_to_inner_kernel(SpinorPtr<32> out, SpinorPtr<64> in,
+                                                          const double2* __restrict__ G1, int n, int stride)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    C G[9], v[12];
-    load9(G1, stride, i, G);
-    SpinorIO<64>::load(in, stride, i, v);
-    Cplx<typename Prec<PO>::R> o[12];
+    const int j = blockIdx.x * blockDim.x + threadIdx.x, H = n / 2;
+    if (j >= H) return;
+    C2 o[12];
 #pragma unroll
-    for (int s = 0; s < 4; ++s)
+    for (int h = 0; h < 2; ++h) {
+        C G[9], v[12];
+        load9(G1, stride, j + h * H, G);
+        SpinorIO<64>::load(in, stride, j + h * H, v);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            C acc = cmk(0.0, 0.0);
+        for (int s = 0; s < 4; ++s)
 #pragma unroll
-            for (int b = 0; b < 3; ++b) cmac(acc, G[3 * a + b], v[3 * s + b]);
-            o[3 * s + a] = {(typename Prec<PO>::R)acc.re, (typename Prec<PO>::R)acc.im};
-        }
-    SpinorIO<PO>::store(out, stride, i, o);
+            for (int a = 0; a < 3; ++a) {
+                C acc = cmk(0.0, 0.0);
+#pragma unroll
+                for (int b = 0; b < 3; ++b) cmac(acc, G[3 * a + b], v[3 * s + b]);
+                if (h == 0) {
+                    o[3 * s + a].re.x = (float)acc.re;
+                    o[3 * s + a].im.x = (float)acc.im;
+                } else {
+                    o[3 * s + a].re.y = (float)acc.re;
+                    o[3 * s + a].im.y = (float)acc.im;
+                }
+            }
+    }
+    SlotF32::store(out.data, stride >> 1, j, o);
 }
 
-// x += G^dagger (xs + alpha p) on the parity-1 sites, xs = 0
+// x += G^dagger (xs + alpha p) on the parity-1 sites, xs = 0; one thread per slot
 template <int PB>
-__global__ void __launch_bounds__(BLAS_THREADS) tg_accumulate_kernel(SpinorPtr<64> x, SpinorPtr<32> xs,
-                                                                     SpinorPtr<PB> p, const SolverScalars* sc,
-                                                                     const double2* __restrict__ G1, int n, int stride)
+__global__ void __launch_bounds__(128) tg_accumulate_kernel(SpinorPtr<64> x, SpinorPtr<32> xs, SpinorPtr<PB> p,
+                                                            const SolverScalars* sc, const double2* __restrict__ G1,
+                                                            int n, int stride)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Cplx<float> b[12];
-    SpinorIO<32>::load(xs, stride, i, b);
+    const int j = blockIdx.x * blockDim.x + threadIdx.x, H = n / 2, ss = stride >> 1;
+    if (j >= H) return;
+    C2 b[12];
+    SlotF32::load(xs.data, ss, j, b);
     if (sc) {
-        Cplx<float> q[12];
-        SpinorIO<PB>::load(p, stride, i, q);
-        const Cplx<float> al = cmk<float>((float)sc->alpha[0], (float)sc->alpha[1]);
+        C2 q[12];
+        slot_load<PB>(p, ss, j, q);
+        const CoefPk al = coef_pk(coef_dev(sc->alpha));
 #pragma unroll
-        for (int k = 0; k < 12; ++k) b[k] = b[k] + cmul(al, q[k]);
+        for (int k = 0; k < 12; ++k) b[k] = caxpy_pk(b[k], al, q[k]);
     }
-    C G[9], a[12];
-    load9(G1, stride, i, G);
-    SpinorIO<64>::load(x, stride, i, a);
 #pragma unroll
-    for (int s = 0; s < 4; ++s)
+    for (int h = 0; h < 2; ++h) {
+        C G[9], a[12];
+        load9(G1, stride, j + h * H, G);
+        SpinorIO<64>::load(x, stride, j + h * H, a);
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
+        for (int s = 0; s < 4; ++s)
 #pragma unroll
-            for (int r = 0; r < 3; ++r)  // (G^dagger)_{c r} = conj(G_{r c})
-                cmacc(a[3 * s + c], G[3 * r + c], cmk((double)b[3 * s + r].re, (double)b[3 * s + r].im));
-    SpinorIO<64>::store(x, stride, i, a);
+            for (int c = 0; c < 3; ++c)
 #pragma unroll
-    for (int k = 0; k < 12; ++k) b[k] = cmk<float>(0.f, 0.f);
-    SpinorIO<32>::store(xs, stride, i, b);
+                for (int r = 0; r < 3; ++r) {  // (G^dagger)_{c r} = conj(G_{r c})
+                    const C2 v = b[3 * s + r];
+                    cmacc(a[3 * s + c], G[3 * r + c],
+                          h == 0 ? cmk((double)v.re.x, (double)v.im.x) : cmk((double)v.re.y, (double)v.im.y));
+                }
+        SpinorIO<64>::store(x, stride, j + h * H, a);
+    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) b[k] = C2{bc2(0.f), bc2(0.f)};
+    SlotF32::store(xs.data, ss, j, b);
 }
 
 }  // namespace
@@ -272,7 +288,7 @@ int tg_to_inner(c2q_ctx* ctx, const c2q_gauge* g, c2q_spinor_eo* out, const c2q_
         return fail(ctx, C2Q_BAD_ARG, "tg_to_inner: FP64 in, FP32 out, transformation built");
     const int n          = in->geom.seo;
     const double2* G1    = static_cast<const double2*>(g->tg_transform.data) + (size_t)9 * g->geom.stride;
-    tg_to_inner_kernel<32><<<(n + BLAS_THREADS - 1) / BLAS_THREADS, BLAS_THREADS, 0, ctx->stream>>>(
+    tg_to_inner_kernel<<<(n / 2 + 127) / 128, 128, 0, ctx->stream>>>(
         sptr<32>(out), sptr<64>(in), G1, n, in->geom.stride);
     ctx->launches++;
     C2Q_CUDA(ctx, cudaGetLastError());
@@ -285,12 +301,12 @@ int tg_accumulate(c2q_ctx* ctx, const c2q_gauge* g, c2q_spinor_eo* x, c2q_spinor
     if (!g->tg_transform.data) return fail(ctx, C2Q_BAD_ARG, "tg_accumulate: transformation not built");
     const int n       = x->geom.seo;
     const double2* G1 = static_cast<const double2*>(g->tg_transform.data) + (size_t)9 * g->geom.stride;
-    const unsigned blocks = (unsigned)((n + BLAS_THREADS - 1) / BLAS_THREADS);
+    const unsigned blocks = (unsigned)((n / 2 + 127) / 128);
     if (p->prec == 16)
-        tg_accumulate_kernel<16><<<blocks, BLAS_THREADS, 0, ctx->stream>>>(sptr<64>(x), sptr<32>(xs), sptr<16>(p),
+        tg_accumulate_kernel<16><<<blocks, 128, 0, ctx->stream>>>(sptr<64>(x), sptr<32>(xs), sptr<16>(p),
                                                                           sc, G1, n, x->geom.stride);
     else
-        tg_accumulate_kernel<32><<<blocks, BLAS_THREADS, 0, ctx->stream>>>(sptr<64>(x), sptr<32>(xs), sptr<32>(p),
+        tg_accumulate_kernel<32><<<blocks, 128, 0, ctx->stream>>>(sptr<64>(x), sptr<32>(xs), sptr<32>(p),
                                                                           sc, G1, n, x->geom.stride);
     ctx->launches++;
     C2Q_CUDA(ctx, cudaGetLastError());
