@@ -5,7 +5,6 @@
 
 #include <cuda_runtime.h>
 
-#include <initializer_list>
 #include <map>
 #include <string>
 #include <vector>
@@ -44,6 +43,9 @@ struct c2q_ctx {
     // staging buffer for AoS host <-> device transfers
     void* staging          = nullptr;
     size_t staging_cap     = 0;
+    // freed blocks of gauge objects by size (link_alloc)
+    std::multimap<size_t, void*> link_cache;
+    size_t link_cached = 0;
     // ring of pinned buffers between pageable host arrays and the device (hostcopy.cu)
     void* hc_ring        = nullptr;
     cudaEvent_t hc_ev[4] = {};
@@ -166,14 +168,19 @@ int gkind_for(int prec, int rec12);
 int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f, bool clear = false);
 void field_free(c2q_spinor_eo* f);
 size_t field_bytes(const Geom& g, int prec);
-// Memory of the gauge objects (links, derived copies, momenta) from the same pool as
-// the spinor fields, in stream order: a program that replaces a gauge field gets
-// the freed blocks back instead of new mappings (some milliseconds of the first solve
-// on a new field).  link_free waits for the device, as other contexts may still read the
-// block, and gives back what the pool holds unused beyond POOL_KEEP.
-constexpr size_t POOL_KEEP = (size_t)22 << 30;  // an eighth of a B200
+// Memory of the gauge objects (links, derived copies, momenta).  A freed block stays
+// with the context for the next request of the same size, so that a program that
+// goes from one gauge field to the next pays for no new mappings and no device-wide
+// frees; at most LINK_KEEP bytes are kept, and all go back when memory runs out or
+// the context ends.  link_free: no kernel may still use the block (link_quiet waits
+// for the device, as other contexts may read a gauge object).
+// (cudaMalloc'ed: the stream-ordered pool maps new memory several times slower,
+// 35 ms against 6 ms for the copies of a first 32^3x64 field.)
+constexpr size_t LINK_KEEP = (size_t)22 << 30;  // an eighth of a B200
 cudaError_t link_alloc(c2q_ctx* ctx, void** p, size_t bytes);
-void link_free(c2q_ctx* ctx, std::initializer_list<void*> blocks);
+void link_free(c2q_ctx* ctx, void* p, size_t bytes);
+void link_trim(c2q_ctx* ctx);
+inline void link_quiet() { cudaDeviceSynchronize(); }
 int gauge_ensure(c2q_gauge* g, int kind);  // builds a lower-precision copy on first use
 // frees every copy derived from the FP64 18-real links (rebuilt on next use)
 int gauge_drop_derived(c2q_gauge* g);

@@ -144,7 +144,13 @@ int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f
         return fail(ctx, C2Q_BAD_ARG, "FP32 / FP16 fields pair the times t and t + NT/2: NT must be a multiple of 4");
     const size_t bytes = field_bytes(f->geom, prec);
     void* p            = nullptr;
-    C2Q_CUDA(ctx, cudaMallocAsync(&p, bytes, ctx->stream));
+    cudaError_t e      = cudaMallocAsync(&p, bytes, ctx->stream);
+    if (e == cudaErrorMemoryAllocation && ctx->link_cached) {
+        cudaGetLastError();
+        link_trim(ctx);
+        e = cudaMallocAsync(&p, bytes, ctx->stream);
+    }
+    C2Q_CUDA(ctx, e);
     if (clear) C2Q_CUDA(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));
     f->data = p;
     f->norm = prec == 16 ? reinterpret_cast<float*>(static_cast<char*>(p) + (size_t)f->geom.stride * 3 * 16) : nullptr;
@@ -368,23 +374,39 @@ __global__ void gauge_convert16_kernel(const double2* __restrict__ in, uint4* __
 
 cudaError_t link_alloc(c2q_ctx* ctx, void** p, size_t bytes)
 {
-    const cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
-    if (e != cudaSuccess) *p = nullptr;
+    *p      = nullptr;
+    auto it = ctx->link_cache.find(bytes);
+    if (it != ctx->link_cache.end()) {
+        *p = it->second;
+        ctx->link_cache.erase(it);
+        ctx->link_cached -= bytes;
+        return cudaSuccess;
+    }
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->link_cached) {
+        cudaGetLastError();
+        link_trim(ctx);
+        e = cudaMalloc(p, bytes);
+    }
     return e;
 }
 
-void link_free(c2q_ctx* ctx, std::initializer_list<void*> blocks)
+void link_free(c2q_ctx* ctx, void* p, size_t bytes)
 {
-    cudaDeviceSynchronize();
-    for (void* p : blocks)
-        if (p) cudaFreeAsync(p, ctx->stream);
-    cudaMemPool_t pool;
-    uint64_t held = 0, used = 0;
-    if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) != cudaSuccess) return;
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return;
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess) return;
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return;
-    if (held > used + POOL_KEEP) cudaMemPoolTrimTo(pool, used + POOL_KEEP);
+    if (!p) return;
+    if (ctx->link_cached + bytes > LINK_KEEP) {
+        cudaFree(p);
+        return;
+    }
+    ctx->link_cache.emplace(bytes, p);
+    ctx->link_cached += bytes;
+}
+
+void link_trim(c2q_ctx* ctx)
+{
+    for (auto& b : ctx->link_cache) cudaFree(b.second);
+    ctx->link_cache.clear();
+    ctx->link_cached = 0;
 }
 
 int gauge_ensure(c2q_gauge* g, int kind)
@@ -411,7 +433,7 @@ int gauge_ensure(c2q_gauge* g, int kind)
         C2Q_CUDA(ctx, link_alloc(ctx, &tmp, lanes * 9 * 16));
         const int rc = tg_links_fp64(g, tmp);
         if (rc) {
-            cudaFreeAsync(tmp, ctx->stream);
+            cudaFree(tmp);
             return rc;
         }
         src = static_cast<const double2*>(tmp);
@@ -419,7 +441,7 @@ int gauge_ensure(c2q_gauge* g, int kind)
     void* p = nullptr;
     const cudaError_t ea = link_alloc(ctx, &p, bytes);
     if (ea != cudaSuccess) {
-        if (tmp) cudaFreeAsync(tmp, ctx->stream);
+        cudaFree(tmp);
         return cuda_fail(ctx, ea, "cudaMalloc(gauge copy)");
     }
     const int threads = 256;
@@ -437,11 +459,11 @@ int gauge_ensure(c2q_gauge* g, int kind)
     }
     ctx->launches++;
     const cudaError_t ek = cudaGetLastError();
-    if (tmp) cudaFreeAsync(tmp, ctx->stream);
-    // (the copy may be read on other streams)
+    // the scratch is free again, and the copy may be read on other streams
     cudaStreamSynchronize(ctx->stream);
+    link_free(ctx, tmp, lanes * 9 * 16);
     if (ek != cudaSuccess) {
-        cudaFreeAsync(p, ctx->stream);
+        cudaFree(p);
         return cuda_fail(ctx, ek, "gauge conversion");
     }
     g->store[kind].data  = p;
@@ -456,10 +478,12 @@ int gauge_drop_derived(c2q_gauge* g)
     for (int k = 1; k < GAUGE_KINDS; ++k) any = any || g->store[k].data;
     C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (!any) return C2Q_OK;
-    link_free(ctx, {g->store[1].data, g->store[2].data, g->store[3].data, g->store[4].data, g->store[5].data,
-                    g->store[6].data, g->store[7].data, g->store[8].data, g->store[9].data, g->tg_transform.data});
-    static_assert(GAUGE_KINDS == 10, "every derived copy is freed above");
-    for (int k = 1; k < GAUGE_KINDS; ++k) g->store[k] = GaugeStore{};
+    link_quiet();
+    for (int k = 1; k < GAUGE_KINDS; ++k) {
+        link_free(ctx, g->store[k].data, g->store[k].bytes);
+        g->store[k] = GaugeStore{};
+    }
+    link_free(ctx, g->tg_transform.data, g->tg_transform.bytes);
     g->tg_transform = GaugeStore{};
     return C2Q_OK;
 }
@@ -883,6 +907,7 @@ C2Q_EXPORT int c2q_ctx_destroy(c2q_ctx* ctx)
     cudaFree(ctx->red_result);
     cudaFree(ctx->scalars);
     cudaFree(ctx->staging);
+    link_trim(ctx);
     if (ctx->hc_ring) cudaFreeHost(ctx->hc_ring);
     for (auto e : ctx->hc_ev)
         if (e) cudaEventDestroy(e);
@@ -976,7 +1001,8 @@ C2Q_EXPORT int c2q_gauge_destroy(c2q_gauge* g)
 {
     if (!g) return C2Q_OK;
     gauge_drop_derived(g);
-    link_free(g->ctx, {g->store[G64].data});
+    link_quiet();
+    link_free(g->ctx, g->store[G64].data, g->store[G64].bytes);
     delete g;
     return C2Q_OK;
 }

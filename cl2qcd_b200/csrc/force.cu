@@ -242,7 +242,7 @@ C2Q_EXPORT int c2q_gaugemomenta_create(c2q_ctx* ctx, const c2q_lattice* lat, c2q
     }
     const cudaError_t e = cudaMemsetAsync(m->data, 0, m->bytes, ctx->stream);
     if (e != cudaSuccess) {
-        cudaFreeAsync(m->data, ctx->stream);
+        cudaFree(m->data);
         delete m;
         return cuda_fail(ctx, e, "cudaMemsetAsync(gauge momenta)");
     }
@@ -253,7 +253,8 @@ C2Q_EXPORT int c2q_gaugemomenta_create(c2q_ctx* ctx, const c2q_lattice* lat, c2q
 C2Q_EXPORT int c2q_gaugemomenta_destroy(c2q_gaugemomenta* m)
 {
     if (!m) return C2Q_OK;
-    link_free(m->ctx, {m->data});
+    link_quiet();
+    link_free(m->ctx, m->data, m->bytes);
     delete m;
     return C2Q_OK;
 }

@@ -253,7 +253,7 @@ int tg_ensure(c2q_gauge* g)
     ctx->launches++;
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
-        cudaFreeAsync(p, ctx->stream);
+        cudaFree(p);
         return cuda_fail(ctx, e, "tg_transform_kernel");
     }
     g->tg_transform.data  = p;
