@@ -250,8 +250,17 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
     const bool small = pcg64_applies(ctx, op, g);
     // Q+Q- with the vector updates in its sweeps
     const bool fused = !small && op == C2Q_OP_QPLUSQMINUS_EO && adjoint_weights(g);
+    double x2 = 0;
+    rc        = norm2(ctx, x, &x2);
+    if (rc) return rc;
+    bool zero_x = x2 == 0.0;  // A x needs no sweeps
     // rn = b - A x, omega = |rn|^2, p = rn
     auto refresh = [&]() -> int {
+        if (zero_x) {
+            zero_x = false;
+            int e  = saxpy_norm(ctx, rn, Cx{0, 0}, b, b, FIN_CG_OMEGA, nullptr);
+            return e ? e : copy_field(ctx, p, rn);
+        }
         DotSpec d;
         d.mode = DOT_RES;
         d.y    = b;
@@ -1402,6 +1411,7 @@ int bicgstab_dev(EoSpace& sp, c2q_spinor_eo* x, c2q_spinor_eo* b, const c2q_solv
         if (!e) e = blas(B_SAXPY, aux, one, aux, none, b, nullptr, 2, FIN_STORE_RESULT);
         return e ? e : read_scalars(ctx, ctx->red_result, 2, tr);
     };
+    double r2_confirmed = -1;  // of the returned solution, when already computed
     // the true-residual confirmation (save variant, rel_tol); unpredicated
     auto confirmed = [&](bool* ok) -> int {
         ctx->halt_dev = nullptr;
@@ -1411,6 +1421,7 @@ int bicgstab_dev(EoSpace& sp, c2q_spinor_eo* x, c2q_spinor_eo* b, const c2q_solv
         const double lim = P->rel_tol > 0 ? std::max(P->rel_tol * P->rel_tol * b2, P->prec > 0 ? P->prec : 0.0)
                                           : P->prec;
         *ok = tr[0] < lim;
+        if (*ok) r2_confirmed = tr[0];
         return e;
     };
 
@@ -1508,7 +1519,9 @@ int bicgstab_dev(EoSpace& sp, c2q_spinor_eo* x, c2q_spinor_eo* b, const c2q_solv
     C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     ctx->halt_dev = nullptr;
     double r2t    = 0;
-    {
+    if (r2_confirmed >= 0) {
+        r2t = r2_confirmed;
+    } else {
         double tr[2] = {0, 0};
         rc           = true_r2(tr);
         if (rc) return rc;
