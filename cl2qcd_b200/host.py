@@ -503,7 +503,7 @@ def perform_inversion(system: System, gf: Gaugefield, source: np.ndarray, params
     (inversion.cpp:98-122, result = M^-1 source)."""
     lib = system.lib
     src = np.ascontiguousarray(source, dtype=np.float64).reshape(-1)
-    out = np.zeros_like(src)
+    out = np.empty_like(src)  # written whole; zeroing it would touch every page first
     p = params.c()
     rep = L.CSolveReport()
     act = L.WILSON if action.lower() == "wilson" else L.TWISTEDMASS
@@ -550,7 +550,7 @@ def inverter_ps_correlator(system: System, gf: Gaugefield, params: SolverParamet
             rc = lib.c2q_perform_inversion_eo_fields(system.h, evens[k].h, odds[k].h, gf.h, src, add.kappa,
                                                      add.mubar, act, C.byref(p), C.byref(rep))
         else:
-            res = np.zeros_like(src)
+            res = np.empty_like(src)
             rc = lib.c2q_perform_inversion_full(system.h, res, gf.h, src, add.kappa, add.mubar, act, C.byref(p),
                                                 C.byref(rep))
             if rc >= 0:
