@@ -225,6 +225,8 @@ int pinned_copy(c2q_ctx* ctx, void* dst, size_t dpitch, const void* src, size_t 
 // Residual ring slot k (n rows of `width` bytes at src, row pitch spitch): into
 // ring_dev on the context's stream, then to the pinned host buffer dst_host_dev
 // (the device alias of a pinned slot) on the monitor stream; ring_ev[k % 4]
+// (src null: a kernel on the stream has filled ring_slot(ctx, k)).
+inline double* ring_slot(c2q_ctx* ctx, int k) { return ctx->ring_dev + (size_t)(k % 4) * 16 * 4; }
 // completes when the host can read it.
 int ring_push(c2q_ctx* ctx, int k, double* dst_host_dev, const void* src, size_t spitch, size_t width, int n);
 int ensure_partials(c2q_ctx* ctx, size_t blocks);

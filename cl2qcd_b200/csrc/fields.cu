@@ -234,8 +234,8 @@ int pinned_copy(c2q_ctx* ctx, void* dst, size_t dpitch, const void* src, size_t 
 int ring_push(c2q_ctx* ctx, int k, double* dst_host_dev, const void* src, size_t spitch, size_t width, int n)
 {
     if (width > 4 * sizeof(double) || n < 1 || n > 16) return fail(ctx, C2Q_BAD_ARG, "ring_push: slot size");
-    double* slot = ctx->ring_dev + (size_t)(k % 4) * 16 * 4;
-    int rc       = pinned_copy(ctx, slot, 4 * sizeof(double), src, spitch, width, n);
+    double* slot = ring_slot(ctx, k);
+    int rc       = src ? pinned_copy(ctx, slot, 4 * sizeof(double), src, spitch, width, n) : C2Q_OK;
     if (rc) return rc;
     C2Q_CUDA(ctx, cudaEventRecord(ctx->mon_ev[k % 4], ctx->stream));
     C2Q_CUDA(ctx, cudaStreamWaitEvent(ctx->monitor, ctx->mon_ev[k % 4], 0));

@@ -1228,11 +1228,21 @@ int bicgstab_generic(S& sp, typename S::V x, typename S::V b, const c2q_solver_p
 // iterate the reference's loop returns.  A stop that needs the host (the
 // true-residual confirmation of the save variant and of rel_tol) clears the
 // halt and re-queues the iteration that was skipped.
-__global__ void bicg_end_kernel(SolverScalars* s)
+// (slot: this iteration's place in the context's residual ring)
+__global__ void bicg_end_kernel(SolverScalars* s, double* slot)
 {
+    pdl_enter();
     if (threadIdx.x != 0) return;
-    s->halt      = s->halt | s->halt_next;  // the next iteration's opening test takes effect
-    s->halt_next = 0;
+    const int halt = s->halt | s->halt_next;  // the next iteration's opening test takes effect
+    s->halt        = halt;
+    s->halt_next   = 0;
+    // resid, aux[2], flag, halt: the first 32 bytes from SolverScalars::resid
+    slot[0]      = s->resid;
+    slot[1]      = s->aux[0];
+    slot[2]      = s->aux[1];
+    int* flags   = reinterpret_cast<int*>(slot + 3);
+    flags[0]     = s->flag;
+    flags[1]     = halt;
 }
 
 struct HaltScope {  // the context's launch predicate for the duration of a solve
@@ -1356,13 +1366,9 @@ struct BicgLoop {
     // ring slot k: resid, aux[2], flag, halt -- the first 32 bytes from SolverScalars::resid
     int push(int k)
     {
-        static_assert(offsetof(SolverScalars, halt) ==
-                          offsetof(SolverScalars, resid) + 3 * sizeof(double) + sizeof(int),
-                      "halt follows resid, aux[2] and flag");
-        bicg_end_kernel<<<1, 32, 0, ctx->stream>>>(sc);
+        C2Q_CUDA(ctx, launch_dep(ctx->pdl, bicg_end_kernel, dim3(1), dim3(32), 0, ctx->stream, sc, ring_slot(ctx, k)));
         ctx->launches++;
-        C2Q_CUDA(ctx, cudaGetLastError());
-        return ring_push(ctx, k, ctx->host_pinned_dev + 32 + 4 * (k % 4), &sc->resid, 0, 4 * sizeof(double), 1);
+        return ring_push(ctx, k, ctx->host_pinned_dev + 32 + 4 * (k % 4), nullptr, 0, 4 * sizeof(double), 1);
     }
     int pop(int k, double* r, int* h)
     {
