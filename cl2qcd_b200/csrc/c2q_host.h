@@ -77,7 +77,6 @@ struct c2q_ctx {
         float us[5];  // per choice; 0 where a choice does not apply to the shape
     };
     std::map<std::vector<int>, TuneEntry> tune;
-    c2q::SolverScalars* tune_scratch = nullptr;  // reductions of tuning launches land here
     bool autotune = true;
     // dependent launches of the solver-loop kernels (launch_dep); environment
     // C2Q_DEPENDENT_LAUNCH=0 turns them off for new contexts
@@ -225,9 +224,9 @@ int pinned_copy(c2q_ctx* ctx, void* dst, size_t dpitch, const void* src, size_t 
 // Residual ring slot k (n rows of `width` bytes at src, row pitch spitch): into
 // ring_dev on the context's stream, then to the pinned host buffer dst_host_dev
 // (the device alias of a pinned slot) on the monitor stream; ring_ev[k % 4]
+// completes when the host can read it.
 // (src null: a kernel on the stream has filled ring_slot(ctx, k)).
 inline double* ring_slot(c2q_ctx* ctx, int k) { return ctx->ring_dev + (size_t)(k % 4) * 16 * 4; }
-// completes when the host can read it.
 int ring_push(c2q_ctx* ctx, int k, double* dst_host_dev, const void* src, size_t spitch, size_t width, int n);
 int ensure_partials(c2q_ctx* ctx, size_t blocks);
 

@@ -83,7 +83,7 @@ int pcg_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B)
     prm.delta  = B.delta;
     prm.first  = B.first;
     prm.iters  = B.iters;
-    int rc     = ensure_partials(ctx, (size_t)prm.ntiles * B.n);
+    int rc     = ensure_partials(ctx, (size_t)prm.ntiles * PK_WARPS * B.n);
     if (rc) return rc;
     prm.partials = ctx->partials;
     prm.ctl      = static_cast<PcgCtl*>(B.ctl);

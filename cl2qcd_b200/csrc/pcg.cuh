@@ -15,8 +15,8 @@
 //
 // The arithmetic, its order and the rule that judges an iteration's residual
 // (one iteration after it, as the host does) are those of the ordinary path, so
-// the iterates are bitwise the same: a reduction leaves one partial per tile,
-// and after the barrier every block adds them up in the order of finish_group
+// the iterates are bitwise the same: a reduction leaves one partial per warp,
+// and after the barrier every block adds them up in the order of pk_finish_kernel
 // and runs the same finisher on its own copy of the solver scalars, which
 // saves the second barrier that one finishing block would need.
 #pragma once
@@ -57,32 +57,45 @@ struct PcgParams : PkStencil {
     int first;          // the solve's first iteration comes first: p is the residual, nothing to judge yet
     unsigned skip;      // bit r: the residual before the first iteration is a true one, not to be judged
     int iters;          // at most
-    double* partials;   // ntiles * nrhs
+    double* partials;   // one per warp, tile and right-hand side
     PcgCtl* ctl;
 };
 
-// The sum of right-hand side rhs's partials, in the order of finish_group and
-// block_sum with PK_THREADS threads, by one warp (valid in lane 0).
-__device__ __forceinline__ double pcg_sum(const double* partials, int ntiles, int nrhs, int rhs)
+// The sums of all right-hand sides' partials (one per warp of each tile) into tot, by
+// the whole block, in the order of pk_finish_kernel: partials j, j + 1024, ... per
+// accumulator j, a tree over each 32 accumulators, a tree over those.
+__device__ __forceinline__ void pcg_sums(const double* partials, int nparts, int nrhs, double* tot, double* smem)
 {
-    static_assert(PK_THREADS == 128, "four warps of block_sum");
-    const int lane = threadIdx.x & 31;
-    double a[4]    = {0.0, 0.0, 0.0, 0.0};
-    for (int m = 0; m < ntiles; m += PK_THREADS) {
-        double t[4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int rhs = 0; rhs < nrhs; ++rhs) {
+        double a[32 / PK_WARPS];
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const int k = m + 32 * w + lane;
-            t[w]        = k < ntiles ? __ldcg(partials + (size_t)k * nrhs + rhs) : 0.0;
+        for (int q = 0; q < 32 / PK_WARPS; ++q) {
+            const int j = 32 * (PK_WARPS * q + warp) + lane;
+            a[q]        = j < nparts ? __ldcg(partials + (size_t)j * nrhs + rhs) : 0.0;
         }
+        for (int m = 1024; m < nparts; m += 1024)
 #pragma unroll
-        for (int w = 0; w < 4; ++w) a[w] += t[w];
+            for (int q = 0; q < 32 / PK_WARPS; ++q) {
+                const int j = m + 32 * (PK_WARPS * q + warp) + lane;
+                if (j < nparts) a[q] += __ldcg(partials + (size_t)j * nrhs + rhs);
+            }
+#pragma unroll
+        for (int q = 0; q < 32 / PK_WARPS; ++q)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) a[q] += __shfl_down_sync(0xffffffffu, a[q], o);
+        if (lane == 0)
+#pragma unroll
+            for (int q = 0; q < 32 / PK_WARPS; ++q) smem[PK_WARPS * q + warp] = a[q];
+        __syncthreads();
+        if (warp == 0) {
+            double t = smem[lane];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+            if (lane == 0) tot[rhs] = t;
+        }
+        __syncthreads();
     }
-#pragma unroll
-    for (int w = 0; w < 4; ++w)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a[w] += __shfl_down_sync(0xffffffffu, a[w], o);
-    return (a[0] + a[2]) + (a[1] + a[3]);
 }
 
 template <int P, int NL>
@@ -93,7 +106,7 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, 0>::MINB) pcg_kerne
     __shared__ SolverScalars sc[PK_MAX_RHS];
     __shared__ double prev[PK_MAX_RHS], maxrr[PK_MAX_RHS], judged[PK_MAX_RHS];
     __shared__ int prev_flag[PK_MAX_RHS], judged_flag[PK_MAX_RHS];
-    __shared__ double smem[32];
+    __shared__ double smem[32], tot[PK_MAX_RHS];
     __shared__ int ok, stop;
     uint4* mine     = ring + threadIdx.x;
     uint4* s8       = mine + (size_t)((8 % S::STAGES) * S::CH) * PK_THREADS;
@@ -190,33 +203,28 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, 0>::MINB) pcg_kerne
                     else if (ph == 3)
                         pk_cg_residual<P, NL>(acc, sc[rhs].alpha, static_cast<float4*>(F.rs), ss, j, s8, s9, dre);
                 }
-                if (axpy) {
-                    double dv[1] = {(double)dre.x + (double)dre.y};
-                    block_sum<1>(dv, smem);
-                    if (threadIdx.x == 0) prm.partials[(size_t)tile * nrhs + rhs] = dv[0];
-                }
+                if (axpy) pk_partial<DOT_SELF>(dre, bc2(0.f), bc2(0.f), prm.partials, tile, nrhs, rhs);
             }
             if (!grid_barrier(&prm.ctl->arrived, &prm.ctl->error, target += gridDim.x, &ok)) return;
             if (axpy) {
-                for (int r = threadIdx.x >> 5; r < nrhs; r += PK_THREADS / 32) {
-                    const double v[2] = {pcg_sum(prm.partials, prm.ntiles, nrhs, r), 0.0};
-                    if ((threadIdx.x & 31) == 0) {
-                        RedArgs ra;
-                        ra.sc  = &sc[r];
-                        ra.fin = ph == 1 ? FIN_CG_ALPHA : FIN_CG_BETA;
-                        finish_apply<2>(ra, v);
-                        if (ph == 3) {
-                            // judge the residual of the iteration before this one
-                            if (!(it == 0 && (prm.first || ((prm.skip >> r) & 1u)))) {
-                                const double q = prev[r], rn = sqrt(q);
-                                judged[r]      = q;
-                                judged_flag[r] = prev_flag[r];
-                                if (rn > maxrr[r]) maxrr[r] = rn;
-                                if (q != q || prev_flag[r] || rn < prm.delta * maxrr[r] || q < prm.f[r].thr) stop = 1;
-                            }
-                            prev[r]      = sc[r].resid;
-                            prev_flag[r] = sc[r].flag;
+                pcg_sums(prm.partials, prm.ntiles * PK_WARPS, nrhs, tot, smem);
+                for (int r = threadIdx.x; r < nrhs; r += PK_THREADS) {
+                    const double v[2] = {tot[r], 0.0};
+                    RedArgs ra;
+                    ra.sc  = &sc[r];
+                    ra.fin = ph == 1 ? FIN_CG_ALPHA : FIN_CG_BETA;
+                    finish_apply<2>(ra, v);
+                    if (ph == 3) {
+                        // judge the residual of the iteration before this one
+                        if (!(it == 0 && (prm.first || ((prm.skip >> r) & 1u)))) {
+                            const double q = prev[r], rn = sqrt(q);
+                            judged[r]      = q;
+                            judged_flag[r] = prev_flag[r];
+                            if (rn > maxrr[r]) maxrr[r] = rn;
+                            if (q != q || prev_flag[r] || rn < prm.delta * maxrr[r] || q < prm.f[r].thr) stop = 1;
                         }
+                        prev[r]      = sc[r].resid;
+                        prev_flag[r] = sc[r].flag;
                     }
                 }
                 __syncthreads();

@@ -74,8 +74,8 @@ static void pk_dispatch(const PkParams<P>& prm, int cfg, int nl, int epi, int do
 // Autotuner: the first launch of each shape (precision, link format,
 // epilogue, reduction, phase pattern, batch size, volume) outside stream
 // capture times every configuration -- one warm-up launch, then two timed
-// launches each, with the reductions redirected to scratch so the caller's
-// solver scalars are untouched -- and keeps the fastest.  The timed launches
+// launches each, of the sweep alone (its reduction's end touches the solver
+// scalars) -- and keeps the fastest.  The timed launches
 // are idempotent (the output depends only on the inputs; the in-place CG
 // residual update is timed as the same sweep without it), so tuning does not
 // change results.  Shapes first met inside a graph capture use
@@ -95,10 +95,66 @@ static bool pk_rb2_applies(const PkParams<P>& prm)
     return P == 16 && prm.tg && prm.nrhs >= 2;
 }
 
-// Launch a sweep with a tuning choice.
-template <int P>
-static int pk_run(c2q_ctx* ctx, const PkParams<P>& prm, int nl, int epi, int dot, int choice, cudaStream_t s)
+// The end of a reducing sweep: right-hand side blockIdx.x's partials added up in a
+// fixed order (thread j takes partials j, j + 1024, ..., then the tree of block_sum)
+// and the solver-scalar finisher.
+constexpr int PK_FINISH_THREADS = 1024;
+struct PkFinish {
+    RedArgs red;
+    SolverScalars* sc[PK_MAX_RHS];
+    int nparts, nrhs, nv;  // nv 1 or 2 numbers per partial
+};
+__global__ void __launch_bounds__(PK_FINISH_THREADS) pk_finish_kernel(const PkFinish A)
 {
+    pdl_enter();
+    if (halted(A.red)) return;
+    __shared__ double smem[2 * 32];
+    const int rhs = blockIdx.x;
+    double v[2]   = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (k >= A.nv) break;
+        const double* p = A.red.partials + (size_t)rhs * A.nv + k;
+        const size_t st = (size_t)A.nrhs * A.nv;
+        for (int m0 = threadIdx.x; m0 < A.nparts; m0 += 8 * PK_FINISH_THREADS) {
+            double t[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int m = m0 + u * PK_FINISH_THREADS;
+                t[u]        = m < A.nparts ? __ldcg(p + m * st) : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[k] += t[u];
+        }
+    }
+    block_sum<2>(v, smem);
+    if (threadIdx.x == 0) {
+        RedArgs ra = A.red;
+        if (A.sc[rhs]) ra.sc = A.sc[rhs];
+        finish_apply<2>(ra, v);
+    }
+}
+
+template <int P>
+static int pk_finish(c2q_ctx* ctx, const PkParams<P>& prm, int dot, cudaStream_t s)
+{
+    PkFinish A;
+    A.red    = prm.red;
+    A.nparts = prm.ntiles * PK_WARPS;
+    A.nrhs   = prm.nrhs;
+    A.nv     = dot == DOT_Y ? 2 : 1;
+    for (int r = 0; r < prm.nrhs; ++r) A.sc[r] = prm.r[r].sc;
+    C2Q_CUDA(ctx, launch_dep(prm.pdl != 0, pk_finish_kernel, dim3(prm.nrhs), dim3(PK_FINISH_THREADS), 0, s, A));
+    ctx->launches++;
+    return C2Q_OK;
+}
+
+// Launch a sweep with a tuning choice, and (finish) its reduction's end.
+template <int P>
+static int pk_run(c2q_ctx* ctx, const PkParams<P>& prm, int nl, int epi, int dot, int choice, cudaStream_t s,
+                  bool finish)
+{
+    finish = finish && dot != DOT_NONE && dot != DOT_XUPD;
     if constexpr (P == 16) {
         if (choice == PK_CHOICE_RB2) {
             const int npair = prm.nrhs / 2;
@@ -106,18 +162,20 @@ static int pk_run(c2q_ctx* ctx, const PkParams<P>& prm, int nl, int epi, int dot
             a.nrhs          = 2 * npair;
             if (!pk2_dispatch(a, nl, epi, dot, prm.ntiles * npair, s))
                 return fail(ctx, C2Q_BAD_ARG, "no two-sources-per-thread sweep for this shape");
+            int rc = finish ? pk_finish<16>(ctx, a, dot, s) : C2Q_OK;
             if (prm.nrhs & 1) {  // the odd last right-hand side, one per thread
                 PkParams<16> b = prm;
                 b.r[0]         = prm.r[prm.nrhs - 1];
                 b.nrhs         = 1;
-                pk_dispatch<16>(b, 0, nl, epi, dot, pk_grid(ctx, 16, nl, 0, false, b.ntiles, 1), s);
+                if (!rc) pk_dispatch<16>(b, 0, nl, epi, dot, pk_grid(ctx, 16, nl, 0, false, b.ntiles, 1), s);
+                if (!rc && finish) rc = pk_finish<16>(ctx, b, dot, s);
             }
-            return C2Q_OK;
+            return rc;
         }
     }
     const int cfg = choice & 1;
     pk_dispatch<P>(prm, cfg, nl, epi, dot, pk_grid(ctx, P, nl, cfg, choice >> 1, prm.ntiles, prm.nrhs), s);
-    return C2Q_OK;
+    return finish ? pk_finish<P>(ctx, prm, dot, s) : C2Q_OK;
 }
 
 template <int P>
@@ -145,25 +203,17 @@ static int pk_choose(c2q_ctx* ctx, const PkParams<P>& prm, int nl, int epi, int 
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     C2Q_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cs));
     if (cs != cudaStreamCaptureStatusNone) return C2Q_OK;
-    if (!ctx->tune_scratch)
-        C2Q_CUDA(ctx, cudaMalloc(&ctx->tune_scratch, (PK_MAX_RHS + 1) * sizeof(SolverScalars)));
     PkParams<P> t = prm;
-    t.red.sc      = ctx->tune_scratch + PK_MAX_RHS;
-    t.red.result  = ctx->tune_scratch[PK_MAX_RHS].aux;
     t.red.halt    = nullptr;  // timing launches always run
-    for (int r = 0; r < t.nrhs; ++r) {
-        t.r[r].sc     = ctx->tune_scratch + r;
-        t.r[r].result = nullptr;
-    }
     c2q_ctx::TuneEntry e{0, {0, 0, 0, 0, 0}};
     float best       = 0;
     const int nchoice = pk_rb2_applies(prm) ? PK_CHOICES + 1 : PK_CHOICES;
     for (int c = 0; c < nchoice; ++c) {
-        int rc = pk_run<P>(ctx, t, nl, epi, dot, c, ctx->stream);
+        int rc = pk_run<P>(ctx, t, nl, epi, dot, c, ctx->stream, false);
         if (rc) return rc;
         C2Q_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
-        pk_run<P>(ctx, t, nl, epi, dot, c, ctx->stream);
-        pk_run<P>(ctx, t, nl, epi, dot, c, ctx->stream);
+        pk_run<P>(ctx, t, nl, epi, dot, c, ctx->stream, false);
+        pk_run<P>(ctx, t, nl, epi, dot, c, ctx->stream, false);
         C2Q_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
         C2Q_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
         C2Q_CUDA(ctx, cudaGetLastError());
@@ -237,7 +287,6 @@ static int pk_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PkBatch&
         fill_field(B.x[r], &R.x, &R.x_norm);
         fill_field(B.y[r], &R.y, &R.y_norm);
         R.sc     = B.sc[r];
-        R.result = nullptr;
     }
     prm.nrhs       = B.n;
     prm.pdl        = ctx->pdl;
@@ -245,8 +294,8 @@ static int pk_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PkBatch&
     prm.e          = B.e;
     prm.out_parity = B.out_parity;
     prm.ntiles = (prm.g.H + PK_THREADS - 1) / PK_THREADS;
-    if (B.dot_mode != DOT_NONE && B.dot_mode != DOT_XUPD) {  // one partial per tile and right-hand side
-        int rc0 = ensure_partials(ctx, (size_t)prm.ntiles * B.n);
+    if (B.dot_mode != DOT_NONE && B.dot_mode != DOT_XUPD) {  // (at most two doubles per warp and right-hand side)
+        int rc0 = ensure_partials(ctx, (size_t)prm.ntiles * PK_WARPS * B.n);
         if (rc0) return rc0;
     }
     prm.red.partials = ctx->partials;
@@ -281,7 +330,7 @@ static int pk_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PkBatch&
         tm.bytes           = (double)ref->geom.seo * (links * lk + B.n * per_rhs);
         cudaEventRecord(tm.a, ctx->stream);
     }
-    rc = pk_run<P>(ctx, prm, nl, B.epi, B.dot_mode, choice, ctx->stream);
+    rc = pk_run<P>(ctx, prm, nl, B.epi, B.dot_mode, choice, ctx->stream, true);
     if (rc) return rc;
     if (ctx->profiling) {
         cudaEventRecord(tm.b, ctx->stream);

@@ -29,10 +29,6 @@
 namespace c2q {
 
 constexpr int PK_THREADS = 128;
-// partials per thread and load round of the sweeps' reduction finisher (4096
-// tiles at 32^3x64: two rounds for the 128 threads of the last block)
-constexpr int PK_FINISH_ROUND = 16;
-
 // Fields of one right-hand side of a batch.
 struct PkRhs {
     void* out;
@@ -44,7 +40,6 @@ struct PkRhs {
     const void* y;        // DOT_Y partner
     const float* y_norm;
     SolverScalars* sc;    // finisher target of this right-hand side
-    double* result;       // FIN_STORE_RESULT target (2 doubles)
 };
 
 struct PkGeom {
@@ -686,6 +681,30 @@ __device__ __forceinline__ void pk_self_dot(const C2 acc[12], float2& dre)
     for (int c = 0; c < 12; ++c) dre = fma2(acc[c].re, acc[c].re, fma2(acc[c].im, acc[c].im, dre));
 }
 
+// A reduction leaves one partial per warp (of DOT_Y two numbers, else one), in slot
+// order; pk_finish_kernel adds them up after the sweep.  Nothing in the sweep
+// waits for it: with a ticket per block, every block stayed on its SM for a fence and
+// an atomic after its last store, 2 us a wave, and the barriers of a block-wide sum
+// kept its warps in step.
+constexpr int PK_WARPS = PK_THREADS / 32;
+template <int DOT>
+__device__ __forceinline__ void pk_partial(float2 dre, float2 dim, float2 dq, double* partials, int tile, int nrhs,
+                                           int rhs)
+{
+    constexpr int NV = DOT == DOT_Y ? 2 : 1;
+    double v[NV];
+    v[0] = (double)dre.x + (double)dre.y;
+    if (NV == 2) v[NV - 1] = ((double)dim.x - (double)dq.x) + ((double)dim.y - (double)dq.y);
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k)
+            partials[(((size_t)tile * PK_WARPS + (threadIdx.x >> 5)) * nrhs + rhs) * NV + k] = v[k];
+}
+
 template <int P, int NL, int EPI, int DOT, int PH, int CFG>
 __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, CFG>::MINB) pdslash_kernel(const PkParams<P> prm)
 {
@@ -702,7 +721,6 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, CFG>::MINB) pdslash
     const int blk   = nrhs == 1 ? (int)blockIdx.x : (int)(blockIdx.x / (unsigned)nrhs);
     const int G     = (int)gridDim.x / nrhs;  // blocks per right-hand side
     const PkRhs& rr = prm.r[rhs];
-    __shared__ double smem[2 * 32];
 
     // tiles of PK_THREADS slots; a block takes tiles blk, blk + G, ... (one
     // tile per block unless the grid is sized to the resident blocks)
@@ -761,19 +779,8 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, CFG>::MINB) pdslash
             pk_cg_solution<P, NL>(rr.sc->alpha, yw, ss, j, s8, s9);
         }
     }
-    if (RED) {  // one partial per tile, in tile order
-        double dv[2] = {(double)dre.x + (double)dre.y,
-                        ((double)dim.x - (double)dq.x) + ((double)dim.y - (double)dq.y)};
-        block_sum<2>(dv, smem);
-        store_partial<2>(dv, prm.red, (size_t)tile * nrhs + rhs);
-    }
+    if (RED) pk_partial<DOT>(dre, dim, dq, prm.red.partials, tile, nrhs, rhs);
     }  // tiles
-    if (RED) {
-        RedArgs ra = prm.red;
-        if (rr.sc) ra.sc = rr.sc;
-        if (rr.result) ra.result = rr.result;
-        finish_group<2, PK_FINISH_ROUND>(ra, smem, rhs, nrhs, prm.ntiles, G);
-    }
 }
 
 }  // namespace c2q

@@ -141,7 +141,6 @@ __global__ void __launch_bounds__(PK_THREADS, Pk2Stage<NL>::MINB) pdslash2_kerne
     const int G     = (int)gridDim.x / npair;  // blocks per pair of right-hand sides
     const PkRhs& r0 = prm.r[2 * pair];
     const PkRhs& r1 = prm.r[2 * pair + 1];
-    __shared__ double smem[2 * 32];
 
     for (int tile = blk; tile < prm.ntiles; tile += G) {
     const int j = tile * T + threadIdx.x;
@@ -277,27 +276,12 @@ __global__ void __launch_bounds__(PK_THREADS, Pk2Stage<NL>::MINB) pdslash2_kerne
         pk2_epilogue<EPI, DOT>(acc0, prm, r0, s8, s9, ss, j, dre[0], dim[0], dq[0]);
         pk2_epilogue<EPI, DOT>(acc1, prm, r1, s8 + S::SPC * T, s9 + S::SPC * T, ss, j, dre[1], dim[1], dq[1]);
     }
-    if (RED) {  // one partial per tile and source, in tile order
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            double dv[2] = {(double)dre[r].x + (double)dre[r].y,
-                            ((double)dim[r].x - (double)dq[r].x) + ((double)dim[r].y - (double)dq[r].y)};
-            block_sum<2>(dv, smem);
-            store_partial<2>(dv, prm.red, (size_t)tile * prm.nrhs + 2 * pair + r);
-        }
-    }
-    }  // tiles
     if (RED) {
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const PkRhs& rr = r ? r1 : r0;
-            RedArgs ra      = prm.red;
-            if (rr.sc) ra.sc = rr.sc;
-            if (rr.result) ra.result = rr.result;
-            if (r) __syncthreads();  // every thread has read the first group's flag before it is set again
-            finish_group<2, PK_FINISH_ROUND>(ra, smem, 2 * pair + r, prm.nrhs, prm.ntiles, G);
-        }
+        for (int r = 0; r < 2; ++r)
+            pk_partial<DOT>(dre[r], dim[r], dq[r], prm.red.partials, tile, prm.nrhs, 2 * pair + r);
     }
+    }  // tiles
 }
 
 }  // namespace c2q
