@@ -78,6 +78,15 @@ __global__ void __launch_bounds__(BLAS_PK_THREADS) blas_pk_kernel(const BlasArgs
     const int ss = A.stride >> 1;
     double dv[4] = {0.0, 0.0, 0.0, 0.0};
     if (j < A.n / 2) {
+        if (A.op == B_COPY && !A.dot) {  // word for word
+            const uint4* p  = static_cast<const uint4*>(A.x.data) + j;
+            uint4* q        = static_cast<uint4*>(A.out.data) + j;
+            constexpr int n = P == 16 ? 6 : 12;
+#pragma unroll
+            for (int L = 0; L < n; ++L) q[(size_t)L * ss] = __ldg(p + (size_t)L * ss);
+            if (P == 16) reinterpret_cast<float2*>(A.out.norm)[j] = __ldg(reinterpret_cast<const float2*>(A.x.norm) + j);
+            return;
+        }
         C2 xv[12], r[12];
         slot_load<P>(A.x, ss, j, xv);
         if (A.op == B_BICG_XR) {

@@ -118,7 +118,8 @@ typedef struct {
     int precision;            /* C2Q_PREC_*: inner arithmetic */
     double reliable_delta;    /* mixed precision: reliable update when |r_inner| < delta * max|r| since the last one (default 0.003) */
     int use_rec12;            /* inner operator uses 12-real links */
-    int use_graph;            /* CG: replay the iterations between residual refreshes as a captured CUDA graph */
+    int use_graph;            /* CG: replay the iterations between residual refreshes as a captured CUDA graph
+                                 (small lattices: one cooperative launch whatever this says) */
     int use_temporal_gauge;   /* mixed precision on QplusQminus_eo: inner iterations on the field in the
                                  temporal gauge (T links the identity but on the last slice), where the
                                  T weights are pure phases and the spatial ones real (default 1) */
@@ -293,7 +294,9 @@ C2Q_EXPORT int c2q_ctx_set_autotune(c2q_ctx* ctx, int enable);
  * launch configuration (choice & 1) with one block per tile (choice >> 1 = 0)
  * or a grid-stride grid (1); 4 = two right-hand sides per thread, for FP16
  * batches of two or more in the temporal gauge (elsewhere choice 0); -1 = the
- * autotuner decides (default).  Every choice gives bitwise the same results. */
+ * autotuner decides (default).  Every choice gives bitwise the same results.  The
+ * mixed-precision CG on QplusQminus_eo of small lattices runs whole iterations in
+ * one cooperative launch (bitwise the same too), which has no choice. */
 C2Q_EXPORT int c2q_ctx_set_sweep_choice(c2q_ctx* ctx, int choice);
 C2Q_EXPORT int c2q_ctx_tune_report(const c2q_ctx* ctx, char* buf, int len);
 /* convert_to_eoprec / convert_from_eoprec (physics/lattices/spinorfield_eo.cpp:372-410):
