@@ -202,6 +202,14 @@ struct PkStage : PkChunks<P, NL> {
     static constexpr int STAGES   = (P == 16 && CFG == 0) ? 3 : 2;
     static constexpr int MINB     = P == 16 ? (CFG == 0 ? 3 : 4) : (CFG == 0 ? 2 : 3);
     static constexpr size_t BYTES = (size_t)STAGES * PkChunks<P, NL>::CH * 16 * PK_THREADS;
+    // Neighbour spinors go through L1 where the resident blocks' rings leave it some
+    // room: other hops of the block find part of them there (FP32 18-real 22^3x36:
+    // CG 14.3 -> 12.8 ms).  FP32 12-real with three blocks has 4 KB left and lost by
+    // it (32^3x64 temporal-gauge sweep 87 -> 112 us), so its copies go past L1.
+    static constexpr size_t SMEM  = 228 * 1024;
+    static constexpr size_t FITS  = SMEM / (BYTES + 1024);
+    static constexpr size_t USED  = (FITS < (size_t)MINB ? FITS : (size_t)MINB) * (BYTES + 1024);
+    static constexpr bool L1      = SMEM - USED >= 32 * 1024;
 };
 
 __device__ __forceinline__ void cp16(uint4* smem, const void* g)
@@ -227,14 +235,19 @@ __device__ __forceinline__ void cp_wait()
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// spinor of `slot` of field (d, norm) -> chunks [0, SPC) of a stage
-template <int P>
+// spinor of `slot` of field (d, norm) -> chunks [0, SPC) of a stage, through L1 or past it
+template <int P, bool L1 = false>
 __device__ __forceinline__ void stage_spinor(uint4* st, const void* d, const float* norm, int ss, int slot)
 {
     const uint4* p  = static_cast<const uint4*>(d) + slot;
     constexpr int n = P == 16 ? 6 : 12;
 #pragma unroll
-    for (int c = 0; c < n; ++c) cp16_l1(st + c * PK_THREADS, p + (size_t)c * ss);
+    for (int c = 0; c < n; ++c) {
+        if (L1)
+            cp16_l1(st + c * PK_THREADS, p + (size_t)c * ss);
+        else
+            cp16(st + c * PK_THREADS, p + (size_t)c * ss);
+    }
     if (P == 16) cp8(st + 6 * PK_THREADS, reinterpret_cast<const float2*>(norm) + slot);
 }
 // link of `slot` of a (parity, mu) group -> chunks [SPC, CH)
@@ -552,7 +565,7 @@ __device__ __forceinline__ void pk_stencil(C2 acc[12], const PkStencil& prm, con
         uint4* st       = mine + (size_t)((q % S::STAGES) * S::CH) * PK_THREADS;
         if constexpr (q < 8) {
             constexpr bool back = q & 1;
-            stage_spinor<P>(st, in, in_norm, ss, nb[q]);
+            stage_spinor<P, S::L1>(st, in, in_norm, ss, nb[q]);
             // temporal gauge: the T links between inner slices are the identity
             if (PH != PH_TG || q >= 2 || (back ? fold_b : fold_f))
                 stage_link<P, NL>(st, (back ? bwd_links : fwd_links) + (size_t)(q >> 1) * grp, ss, back ? nb[q] : j);

@@ -184,8 +184,8 @@ __global__ void __launch_bounds__(PK_THREADS, Pk2Stage<NL>::MINB) pdslash2_kerne
             uint4* st       = mine + (size_t)((q % S::STAGES) * S::CH) * T;
             if constexpr (q < 8) {
                 constexpr bool back = q & 1;
-                stage_spinor<16>(st, r0.in, r0.in_norm, ss, nb[q]);
-                stage_spinor<16>(st + S::SPC * T, r1.in, r1.in_norm, ss, nb[q]);
+                stage_spinor<16, true>(st, r0.in, r0.in_norm, ss, nb[q]);
+                stage_spinor<16, true>(st + S::SPC * T, r1.in, r1.in_norm, ss, nb[q]);
                 // temporal gauge: the T links between inner slices are the identity
                 if (q >= 2 || (back ? fold_b : fold_f))
                     stage_link<16, NL>(st + S::SPC * T, (back ? bwd_links : fwd_links) + (size_t)(q >> 1) * grp, ss,
