@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <map>
 #include <string>
 #include <vector>
@@ -43,9 +44,12 @@ struct c2q_ctx {
     // staging buffer for AoS host <-> device transfers
     void* staging          = nullptr;
     size_t staging_cap     = 0;
-    // freed blocks of gauge objects by size (link_alloc)
-    std::multimap<size_t, void*> link_cache;
-    size_t link_cached = 0;
+    // freed blocks of gauge objects (link_free; guarded by that file's mutex)
+    struct LinkBlock {
+        void* p      = nullptr;
+        size_t bytes = 0;
+    };
+    LinkBlock link_cache[32];
     // ring of pinned buffers between pageable host arrays and the device (hostcopy.cu)
     void* hc_ring        = nullptr;
     cudaEvent_t hc_ev[4] = {};
@@ -109,6 +113,8 @@ struct c2q_gauge {
     double tg_lam_re = 1.0, tg_lam_im = 0.0;
     // max |row 2 - conj(row0 x row1)| of the uploaded links (-1: not measured yet)
     double rec12_dev = -1.0;
+    // a context other than its own has queued work on it (gauge_reader)
+    mutable std::atomic<bool> foreign{false};
 };
 
 struct c2q_spinor_eo {
@@ -170,16 +176,28 @@ size_t field_bytes(const Geom& g, int prec);
 // Memory of the gauge objects (links, derived copies, momenta).  A freed block stays
 // with the context for the next request of the same size, so that a program that
 // goes from one gauge field to the next pays for no new mappings and no device-wide
-// frees; at most LINK_KEEP bytes are kept, and all go back when memory runs out or
-// the context ends.  link_free: no kernel may still use the block (link_quiet waits
-// for the device, as other contexts may read a gauge object).
+// frees; at most LINK_KEEP bytes are kept by all contexts of the process together, and
+// all of a context's go back when it ends.  link_free keeps a block only if `quiet`:
+// no kernel may still use it; else it is freed, which waits for the device.
+// Any thread may call these for any context (a solve on one context builds the copies
+// of another's gauge field).
 // (cudaMalloc'ed: the stream-ordered pool maps new memory several times slower,
 // 35 ms against 6 ms for the copies of a first 32^3x64 field.)
 constexpr size_t LINK_KEEP = (size_t)22 << 30;  // an eighth of a B200
 cudaError_t link_alloc(c2q_ctx* ctx, void** p, size_t bytes);
-void link_free(c2q_ctx* ctx, void* p, size_t bytes);
-void link_trim(c2q_ctx* ctx);
-inline void link_quiet() { cudaDeviceSynchronize(); }
+void link_free(c2q_ctx* ctx, void* p, size_t bytes, bool quiet);
+size_t link_trim(c2q_ctx* ctx);  // gives the kept blocks back; their bytes
+// Waits for the context's stream; whether nothing can use an object's memory any more.
+// (Not for the device: a device is not to be synchronised while another thread captures
+// a stream of it.)
+inline bool stream_quiet(c2q_ctx* ctx) { return cudaStreamSynchronize(ctx->stream) == cudaSuccess; }
+// Called where work of `ctx` that reads the links is queued: the block of a field that
+// other contexts have read is not recycled (waiting for its own stream says nothing
+// about theirs).
+inline void gauge_reader(const c2q_gauge* g, const c2q_ctx* ctx)
+{
+    if (g->ctx != ctx) g->foreign.store(true, std::memory_order_relaxed);
+}
 int gauge_ensure(c2q_gauge* g, int kind);  // builds a lower-precision copy on first use
 // frees every copy derived from the FP64 18-real links (rebuilt on next use)
 int gauge_drop_derived(c2q_gauge* g);

@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "blas_pk.cuh"
@@ -145,9 +146,8 @@ int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f
     const size_t bytes = field_bytes(f->geom, prec);
     void* p            = nullptr;
     cudaError_t e      = cudaMallocAsync(&p, bytes, ctx->stream);
-    if (e == cudaErrorMemoryAllocation && ctx->link_cached) {
+    if (e == cudaErrorMemoryAllocation && link_trim(ctx)) {
         cudaGetLastError();
-        link_trim(ctx);
         e = cudaMallocAsync(&p, bytes, ctx->stream);
     }
     C2Q_CUDA(ctx, e);
@@ -372,41 +372,59 @@ __global__ void gauge_convert16_kernel(const double2* __restrict__ in, uint4* __
     }
 }
 
+// the blocks kept by every context, and their bytes
+static std::mutex link_mutex;
+static size_t link_total = 0;
+
 cudaError_t link_alloc(c2q_ctx* ctx, void** p, size_t bytes)
 {
-    *p      = nullptr;
-    auto it = ctx->link_cache.find(bytes);
-    if (it != ctx->link_cache.end()) {
-        *p = it->second;
-        ctx->link_cache.erase(it);
-        ctx->link_cached -= bytes;
-        return cudaSuccess;
+    *p = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(link_mutex);
+        for (auto& b : ctx->link_cache)
+            if (b.p && b.bytes == bytes) {
+                *p = b.p;
+                b  = {};
+                link_total -= bytes;
+                return cudaSuccess;
+            }
     }
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && ctx->link_cached) {
+    if (e == cudaErrorMemoryAllocation && link_trim(ctx)) {
         cudaGetLastError();
-        link_trim(ctx);
         e = cudaMalloc(p, bytes);
     }
     return e;
 }
 
-void link_free(c2q_ctx* ctx, void* p, size_t bytes)
+void link_free(c2q_ctx* ctx, void* p, size_t bytes, bool quiet)
 {
     if (!p) return;
-    if (ctx->link_cached + bytes > LINK_KEEP) {
-        cudaFree(p);
-        return;
+    if (quiet) {
+        std::lock_guard<std::mutex> lk(link_mutex);
+        if (link_total + bytes <= LINK_KEEP)
+            for (auto& b : ctx->link_cache)
+                if (!b.p) {
+                    b = {p, bytes};
+                    link_total += bytes;
+                    return;
+                }
     }
-    ctx->link_cache.emplace(bytes, p);
-    ctx->link_cached += bytes;
+    cudaFree(p);
 }
 
-void link_trim(c2q_ctx* ctx)
+size_t link_trim(c2q_ctx* ctx)
 {
-    for (auto& b : ctx->link_cache) cudaFree(b.second);
-    ctx->link_cache.clear();
-    ctx->link_cached = 0;
+    std::lock_guard<std::mutex> lk(link_mutex);
+    size_t freed = 0;
+    for (auto& b : ctx->link_cache)
+        if (b.p) {
+            cudaFree(b.p);
+            freed += b.bytes;
+            b = {};
+        }
+    link_total -= freed;
+    return freed;
 }
 
 int gauge_ensure(c2q_gauge* g, int kind)
@@ -460,8 +478,7 @@ int gauge_ensure(c2q_gauge* g, int kind)
     ctx->launches++;
     const cudaError_t ek = cudaGetLastError();
     // the scratch is free again, and the copy may be read on other streams
-    cudaStreamSynchronize(ctx->stream);
-    link_free(ctx, tmp, lanes * 9 * 16);
+    link_free(ctx, tmp, lanes * 9 * 16, stream_quiet(ctx));
     if (ek != cudaSuccess) {
         cudaFree(p);
         return cuda_fail(ctx, ek, "gauge conversion");
@@ -471,20 +488,23 @@ int gauge_ensure(c2q_gauge* g, int kind)
     return C2Q_OK;
 }
 
-int gauge_drop_derived(c2q_gauge* g)
+// all of the object's stores from `first` on, and the transformation
+static void gauge_release(c2q_gauge* g, int first)
 {
-    c2q_ctx* ctx = g->ctx;
-    bool any = g->tg_transform.data != nullptr;
-    for (int k = 1; k < GAUGE_KINDS; ++k) any = any || g->store[k].data;
-    C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (!any) return C2Q_OK;
-    link_quiet();
-    for (int k = 1; k < GAUGE_KINDS; ++k) {
-        link_free(ctx, g->store[k].data, g->store[k].bytes);
+    c2q_ctx* ctx     = g->ctx;
+    const bool quiet = stream_quiet(ctx) && !g->foreign.load(std::memory_order_relaxed);
+    for (int k = first; k < GAUGE_KINDS; ++k) {
+        link_free(ctx, g->store[k].data, g->store[k].bytes, quiet);
         g->store[k] = GaugeStore{};
     }
-    link_free(ctx, g->tg_transform.data, g->tg_transform.bytes);
+    link_free(ctx, g->tg_transform.data, g->tg_transform.bytes, quiet);
     g->tg_transform = GaugeStore{};
+}
+
+int gauge_drop_derived(c2q_gauge* g)
+{
+    C2Q_CUDA(g->ctx, cudaStreamSynchronize(g->ctx->stream));
+    gauge_release(g, G64 + 1);
     return C2Q_OK;
 }
 
@@ -588,6 +608,7 @@ int launch_dslash(c2q_ctx* ctx, const c2q_gauge* g, int gkind, c2q_spinor_eo* ou
     if (!same_lattice(out->lat, in->lat) || !same_lattice(out->lat, g->lat))
         return fail(ctx, C2Q_BAD_ARG, "lattice mismatch between fields and gauge field");
     if (!gauge_matches(out->prec, gkind)) return fail(ctx, C2Q_BAD_ARG, "gauge precision mismatch");
+    gauge_reader(g, ctx);
     int rc = gauge_ensure(const_cast<c2q_gauge*>(g), gkind);
     if (rc) return rc;
     if (out->prec == 64) {
@@ -999,9 +1020,7 @@ C2Q_EXPORT int c2q_gauge_create(c2q_ctx* ctx, const c2q_lattice* lat, c2q_gauge*
 C2Q_EXPORT int c2q_gauge_destroy(c2q_gauge* g)
 {
     if (!g) return C2Q_OK;
-    gauge_drop_derived(g);
-    link_quiet();
-    link_free(g->ctx, g->store[G64].data, g->store[G64].bytes);
+    gauge_release(g, G64);
     delete g;
     return C2Q_OK;
 }

@@ -253,8 +253,7 @@ C2Q_EXPORT int c2q_gaugemomenta_create(c2q_ctx* ctx, const c2q_lattice* lat, c2q
 C2Q_EXPORT int c2q_gaugemomenta_destroy(c2q_gaugemomenta* m)
 {
     if (!m) return C2Q_OK;
-    link_quiet();
-    link_free(m->ctx, m->data, m->bytes);
+    link_free(m->ctx, m->data, m->bytes, stream_quiet(m->ctx));  // only its own context works on it
     delete m;
     return C2Q_OK;
 }
@@ -333,6 +332,7 @@ C2Q_EXPORT int c2q_fermion_force_eo(c2q_gaugemomenta* m, const c2q_gauge* g, con
     if (Y == X) return fail(ctx, C2Q_BAD_ARG, "Y and X live on different parities");
     if (evenodd != C2Q_ODD && evenodd != C2Q_EVEN) return fail(ctx, C2Q_BAD_ARG, "evenodd must be ODD or EVEN");
     if (!g->store[G64].data) return fail(ctx, C2Q_BAD_ARG, "gauge field not uploaded");
+    gauge_reader(g, ctx);
     ForceCoef fc;
     // the boundary phases e^{i theta pi / N} with the reference's rounding, without
     // the chemical potential (which multiplies the T link here)

@@ -52,6 +52,7 @@ static int pcg_go(c2q_ctx* ctx, PcgParams& prm)
 
 int pcg_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B)
 {
+    gauge_reader(g, ctx);
     PcgParams prm;
     memset(&prm, 0, sizeof prm);
     const c2q_spinor_eo* ref = B.p[0];

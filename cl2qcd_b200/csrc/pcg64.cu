@@ -323,6 +323,7 @@ bool pcg64_applies(const c2q_ctx* ctx, int op, const c2q_gauge* gf)
 
 int pcg64_run(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const Pcg64Solve& S, Pcg64Result* out)
 {
+    gauge_reader(g, ctx);
     int rc = gauge_ensure(const_cast<c2q_gauge*>(g), gkind);
     if (rc) return rc;
     Params64 prm;

@@ -372,6 +372,7 @@ int launch_pdslash(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PkBatch& B
         if (!(c == 0 || c == 3 || c == 6 || c == 8 || c == 9 || c == 10 || c == 11))
             return fail(ctx, C2Q_BAD_ARG, "no temporal-gauge sweep with this epilogue and reduction");
     }
+    gauge_reader(g, ctx);
     int rc = gauge_ensure(const_cast<c2q_gauge*>(g), gkind);
     if (rc) return rc;
     return P == 32 ? pk_launch<32>(ctx, g, gkind, B) : pk_launch<16>(ctx, g, gkind, B);

@@ -286,6 +286,7 @@ int tg_to_inner(c2q_ctx* ctx, const c2q_gauge* g, c2q_spinor_eo* out, const c2q_
 {
     if (!g->tg_transform.data || out->prec != 32 || in->prec != 64)
         return fail(ctx, C2Q_BAD_ARG, "tg_to_inner: FP64 in, FP32 out, transformation built");
+    gauge_reader(g, ctx);
     const int n          = in->geom.seo;
     const double2* G1    = static_cast<const double2*>(g->tg_transform.data) + (size_t)9 * g->geom.stride;
     tg_to_inner_kernel<<<(n / 2 + 127) / 128, 128, 0, ctx->stream>>>(
@@ -299,6 +300,7 @@ int tg_accumulate(c2q_ctx* ctx, const c2q_gauge* g, c2q_spinor_eo* x, c2q_spinor
                   const SolverScalars* sc)
 {
     if (!g->tg_transform.data) return fail(ctx, C2Q_BAD_ARG, "tg_accumulate: transformation not built");
+    gauge_reader(g, ctx);
     const int n       = x->geom.seo;
     const double2* G1 = static_cast<const double2*>(g->tg_transform.data) + (size_t)9 * g->geom.stride;
     const unsigned blocks = (unsigned)((n / 2 + 127) / 128);
