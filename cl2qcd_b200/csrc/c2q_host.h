@@ -50,6 +50,7 @@ struct c2q_ctx {
         size_t bytes = 0;
     };
     LinkBlock link_cache[32];
+    c2q_ctx* next_ctx = nullptr;  // the process's contexts (also under that mutex)
     // ring of pinned buffers between pageable host arrays and the device (hostcopy.cu)
     void* hc_ring        = nullptr;
     cudaEvent_t hc_ev[4] = {};
@@ -176,9 +177,11 @@ size_t field_bytes(const Geom& g, int prec);
 // Memory of the gauge objects (links, derived copies, momenta).  A freed block stays
 // with the context for the next request of the same size, so that a program that
 // goes from one gauge field to the next pays for no new mappings and no device-wide
-// frees; at most LINK_KEEP bytes are kept by all contexts of the process together, and
-// all of a context's go back when it ends.  link_free keeps a block only if `quiet`:
-// no kernel may still use it; else it is freed, which waits for the device.
+// frees; at most LINK_KEEP bytes are kept by all contexts of the process together.  All
+// go back when any device allocation of the library finds no memory (device_alloc),
+// before a server takes its budget from what is free, and a context's when it ends or
+// is asked (c2q_ctx_trim).  link_free keeps a block only if `quiet`: no kernel may
+// still use it; else it is freed, which waits for the device.
 // Any thread may call these for any context (a solve on one context builds the copies
 // of another's gauge field).
 // (cudaMalloc'ed: the stream-ordered pool maps new memory several times slower,
@@ -187,6 +190,11 @@ constexpr size_t LINK_KEEP = (size_t)22 << 30;  // an eighth of a B200
 cudaError_t link_alloc(c2q_ctx* ctx, void** p, size_t bytes);
 void link_free(c2q_ctx* ctx, void* p, size_t bytes, bool quiet);
 size_t link_trim(c2q_ctx* ctx);  // gives the kept blocks back; their bytes
+size_t link_trim_device(int device);  // those of every context on the device
+// cudaMalloc, and cudaMallocAsync on the context's stream; where memory has run out,
+// once more after every context's kept blocks and the pool's unused memory went back
+cudaError_t device_alloc(c2q_ctx* ctx, void** p, size_t bytes);
+cudaError_t device_alloc_async(c2q_ctx* ctx, void** p, size_t bytes);
 // Waits for the context's stream; whether nothing can use an object's memory any more.
 // (Not for the device: a device is not to be synchronised while another thread captures
 // a stream of it.)

@@ -145,12 +145,7 @@ int field_alloc(c2q_ctx* ctx, const c2q_lattice& lat, int prec, c2q_spinor_eo* f
         return fail(ctx, C2Q_BAD_ARG, "FP32 / FP16 fields pair the times t and t + NT/2: NT must be a multiple of 4");
     const size_t bytes = field_bytes(f->geom, prec);
     void* p            = nullptr;
-    cudaError_t e      = cudaMallocAsync(&p, bytes, ctx->stream);
-    if (e == cudaErrorMemoryAllocation && link_trim(ctx)) {
-        cudaGetLastError();
-        e = cudaMallocAsync(&p, bytes, ctx->stream);
-    }
-    C2Q_CUDA(ctx, e);
+    C2Q_CUDA(ctx, device_alloc_async(ctx, &p, bytes));
     if (clear) C2Q_CUDA(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));
     f->data = p;
     f->norm = prec == 16 ? reinterpret_cast<float*>(static_cast<char*>(p) + (size_t)f->geom.stride * 3 * 16) : nullptr;
@@ -189,9 +184,10 @@ int ensure_staging(c2q_ctx* ctx, size_t bytes)
     if (ctx->staging) {
         C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         cudaFree(ctx->staging);
-        ctx->staging = nullptr;
+        ctx->staging     = nullptr;
+        ctx->staging_cap = 0;
     }
-    C2Q_CUDA(ctx, cudaMalloc(&ctx->staging, bytes));
+    C2Q_CUDA(ctx, device_alloc(ctx, &ctx->staging, bytes));
     ctx->staging_cap = bytes;
     return C2Q_OK;
 }
@@ -203,10 +199,11 @@ int ensure_partials(c2q_ctx* ctx, size_t blocks)
     if (ctx->partials) {
         C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         cudaFree(ctx->partials);
-        ctx->partials = nullptr;
+        ctx->partials     = nullptr;
+        ctx->partials_cap = 0;
     }
     const size_t cap = need < 4096 ? 4096 : need;
-    C2Q_CUDA(ctx, cudaMalloc(&ctx->partials, cap * sizeof(double)));
+    C2Q_CUDA(ctx, device_alloc(ctx, (void**)&ctx->partials, cap * sizeof(double)));
     ctx->partials_cap = cap;
     return C2Q_OK;
 }
@@ -372,9 +369,10 @@ __global__ void gauge_convert16_kernel(const double2* __restrict__ in, uint4* __
     }
 }
 
-// the blocks kept by every context, and their bytes
+// the contexts, the bytes of the blocks they keep, and what guards both
 static std::mutex link_mutex;
-static size_t link_total = 0;
+static c2q_ctx* link_ctxs = nullptr;
+static size_t link_total  = 0;
 
 cudaError_t link_alloc(c2q_ctx* ctx, void** p, size_t bytes)
 {
@@ -389,12 +387,7 @@ cudaError_t link_alloc(c2q_ctx* ctx, void** p, size_t bytes)
                 return cudaSuccess;
             }
     }
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && link_trim(ctx)) {
-        cudaGetLastError();
-        e = cudaMalloc(p, bytes);
-    }
-    return e;
+    return device_alloc(ctx, p, bytes);
 }
 
 void link_free(c2q_ctx* ctx, void* p, size_t bytes, bool quiet)
@@ -413,9 +406,8 @@ void link_free(c2q_ctx* ctx, void* p, size_t bytes, bool quiet)
     cudaFree(p);
 }
 
-size_t link_trim(c2q_ctx* ctx)
+static size_t trim_locked(c2q_ctx* ctx)
 {
-    std::lock_guard<std::mutex> lk(link_mutex);
     size_t freed = 0;
     for (auto& b : ctx->link_cache)
         if (b.p) {
@@ -425,6 +417,53 @@ size_t link_trim(c2q_ctx* ctx)
         }
     link_total -= freed;
     return freed;
+}
+
+size_t link_trim(c2q_ctx* ctx)
+{
+    std::lock_guard<std::mutex> lk(link_mutex);
+    return trim_locked(ctx);
+}
+
+size_t link_trim_device(int device)
+{
+    std::lock_guard<std::mutex> lk(link_mutex);
+    size_t freed = 0;
+    for (c2q_ctx* c = link_ctxs; c; c = c->next_ctx)
+        if (c->device == device) freed += trim_locked(c);
+    return freed;
+}
+
+// the unused memory of the device's stream-ordered pool goes back
+static void pool_trim(int device)
+{
+    cudaMemPool_t pool;
+    if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+}
+
+// The error is the caller's to report, not the next launch check's.
+static cudaError_t reported(cudaError_t e)
+{
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return e;
+}
+
+cudaError_t device_alloc(c2q_ctx* ctx, void** p, size_t bytes)
+{
+    const cudaError_t e = reported(cudaMalloc(p, bytes));
+    if (e != cudaErrorMemoryAllocation) return e;
+    link_trim_device(ctx->device);
+    pool_trim(ctx->device);
+    return reported(cudaMalloc(p, bytes));
+}
+
+cudaError_t device_alloc_async(c2q_ctx* ctx, void** p, size_t bytes)
+{
+    const cudaError_t e = reported(cudaMallocAsync(p, bytes, ctx->stream));
+    if (e != cudaErrorMemoryAllocation) return e;
+    link_trim_device(ctx->device);
+    pool_trim(ctx->device);
+    return reported(cudaMallocAsync(p, bytes, ctx->stream));
 }
 
 int gauge_ensure(c2q_gauge* g, int kind)
@@ -882,9 +921,9 @@ C2Q_EXPORT int c2q_ctx_create(c2q_ctx** out, int device, void* cuda_stream)
         chk(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "cudaStreamCreate");
         ctx->own_stream = true;
     }
-    chk(cudaMalloc(&ctx->ticket, 64 * sizeof(unsigned)), "cudaMalloc(ticket)");
-    chk(cudaMalloc(&ctx->red_result, 8 * sizeof(double)), "cudaMalloc(result)");
-    chk(cudaMalloc(&ctx->scalars, sizeof(SolverScalars)), "cudaMalloc(scalars)");
+    chk(device_alloc(ctx, (void**)&ctx->ticket, 64 * sizeof(unsigned)), "cudaMalloc(ticket)");
+    chk(device_alloc(ctx, (void**)&ctx->red_result, 8 * sizeof(double)), "cudaMalloc(result)");
+    chk(device_alloc(ctx, (void**)&ctx->scalars, sizeof(SolverScalars)), "cudaMalloc(scalars)");
     chk(cudaMallocHost(&ctx->host_pinned, 64 * sizeof(double)), "cudaMallocHost");
     if (rc == C2Q_OK) chk(cudaHostGetDevicePointer((void**)&ctx->host_pinned_dev, ctx->host_pinned, 0),
                           "cudaHostGetDevicePointer");
@@ -893,7 +932,7 @@ C2Q_EXPORT int c2q_ctx_create(c2q_ctx** out, int device, void* cuda_stream)
     for (auto& e : ctx->ring_ev) chk(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
     for (auto& e : ctx->mon_ev) chk(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
     chk(cudaStreamCreateWithFlags(&ctx->monitor, cudaStreamNonBlocking), "cudaStreamCreate(monitor)");
-    chk(cudaMalloc(&ctx->ring_dev, 4 * 16 * 4 * sizeof(double)), "cudaMalloc(ring)");
+    chk(device_alloc(ctx, (void**)&ctx->ring_dev, 4 * 16 * 4 * sizeof(double)), "cudaMalloc(ring)");
     if (rc == C2Q_OK) {
         chk(cudaMemsetAsync(ctx->ticket, 0, 64 * sizeof(unsigned), ctx->stream), "memset");
         chk(cudaMemsetAsync(ctx->scalars, 0, sizeof(SolverScalars), ctx->stream), "memset");
@@ -910,7 +949,22 @@ C2Q_EXPORT int c2q_ctx_create(c2q_ctx** out, int device, void* cuda_stream)
         c2q_ctx_destroy(ctx);
         return rc;
     }
+    {
+        std::lock_guard<std::mutex> lk(link_mutex);
+        ctx->next_ctx = link_ctxs;
+        link_ctxs     = ctx;
+    }
     *out = ctx;
+    return C2Q_OK;
+}
+
+C2Q_EXPORT int c2q_ctx_trim(c2q_ctx* ctx, size_t* bytes)
+{
+    if (!ctx) return C2Q_BAD_ARG;
+    C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    const size_t freed = link_trim(ctx);
+    pool_trim(ctx->device);
+    if (bytes) *bytes = freed;
     return C2Q_OK;
 }
 
@@ -927,7 +981,15 @@ C2Q_EXPORT int c2q_ctx_destroy(c2q_ctx* ctx)
     cudaFree(ctx->red_result);
     cudaFree(ctx->scalars);
     cudaFree(ctx->staging);
-    link_trim(ctx);
+    {
+        std::lock_guard<std::mutex> lk(link_mutex);
+        trim_locked(ctx);
+        for (c2q_ctx** c = &link_ctxs; *c; c = &(*c)->next_ctx)
+            if (*c == ctx) {
+                *c = ctx->next_ctx;
+                break;
+            }
+    }
     if (ctx->hc_ring) cudaFreeHost(ctx->hc_ring);
     for (auto e : ctx->hc_ev)
         if (e) cudaEventDestroy(e);

@@ -228,6 +228,7 @@ C2Q_EXPORT int c2q_server_create(c2q_server** out, int device, int slots, size_t
     if (hbm_budget == 0) {  // 85% of what is free now
         size_t fr = 0, tot = 0;
         cudaSetDevice(device);
+        link_trim_device(device);  // what other contexts keep of freed gauge objects is free
         if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
             c2q_ctx_destroy(loader);
             return C2Q_CUDA_ERROR;
@@ -281,8 +282,10 @@ C2Q_EXPORT int c2q_server_add_gauge(c2q_server* s, unsigned long long gauge_id, 
     if (!rc) rc = c2q_ctx_synchronize(s->loader);
     if (rc) {
         if (g) c2q_gauge_destroy(g);
+        link_trim(s->loader);
         return rc;
     }
+    link_trim(s->loader);  // scratch of the copies: the budget counts gauge fields and requests only
     std::lock_guard<std::mutex> lk(s->m);
     GaugeEntry e{g, c2q_gauge_device_bytes(g)};
     s->gauges[gauge_id] = e;

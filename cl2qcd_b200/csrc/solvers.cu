@@ -628,7 +628,7 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
     if (!rc) rc = gauge_ensure(const_cast<c2q_gauge*>(g), gk64);
     if (rc) return rc;
     SolverScalars* dsc = nullptr;
-    C2Q_CUDA(ctx, cudaMallocAsync(&dsc, n * sizeof(SolverScalars) + pcg_ctl_bytes(), ctx->stream));
+    C2Q_CUDA(ctx, device_alloc_async(ctx, (void**)&dsc, n * sizeof(SolverScalars) + pcg_ctl_bytes()));
     struct Free {
         c2q_ctx* c;
         void* q;

@@ -84,6 +84,12 @@ class System:
     def synchronize(self):
         _check(self.lib.c2q_ctx_synchronize(self.h), self.h, self.lib)
 
+    def trim(self) -> int:
+        """Give back the device memory kept for reuse; the bytes of kept gauge objects' blocks."""
+        n = C.c_size_t()
+        _check(self.lib.c2q_ctx_trim(self.h, C.byref(n)), self.h, self.lib)
+        return n.value
+
     @property
     def launch_count(self) -> int:
         return self.lib.c2q_ctx_launch_count(self.h)

@@ -207,6 +207,11 @@ C2Q_EXPORT int c2q_ctx_create(c2q_ctx** out, int device, void* cuda_stream);
 C2Q_EXPORT int c2q_ctx_destroy(c2q_ctx* ctx);
 C2Q_EXPORT const char* c2q_last_error(const c2q_ctx* ctx);
 C2Q_EXPORT int c2q_ctx_synchronize(c2q_ctx* ctx);
+/* Gives back device memory that the context keeps for reuse: blocks of destroyed gauge
+ * objects (their bytes into *bytes, which may be null) and the unused part of the
+ * device's stream-ordered pool.  The library does this by itself where one of its own
+ * allocations finds no memory; a program calls it before other libraries allocate. */
+C2Q_EXPORT int c2q_ctx_trim(c2q_ctx* ctx, size_t* bytes);
 /* Kernels this library launched on the context since creation (all of them are this library's own). */
 C2Q_EXPORT long long c2q_ctx_launch_count(const c2q_ctx* ctx);
 /* Per-launch timing of the dslash sweeps with CUDA events on the context's

@@ -96,3 +96,91 @@ def test_contexts_in_threads():
     for t in ts:
         t.join()
     assert not err, err
+
+
+class _Reserve:
+    """All free device memory but `keep` bytes, held by another library."""
+
+    def __init__(self, keep):
+        import torch
+        torch.cuda.empty_cache()
+        self.t = torch.empty(torch.cuda.mem_get_info()[0] - keep, dtype=torch.uint8, device="cuda")
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        import torch
+        self.t = None
+        torch.cuda.empty_cache()
+
+
+def test_kept_blocks_serve_other_contexts():
+    """A field and its staging buffer fit although another context keeps what is missing."""
+    import cl2qcd_b200 as c2q
+    a, b = c2q.System(0), c2q.System(0)
+    gfs = [c2q.Gaugefield(a, c2q.Lattice(24, 48)) for _ in range(3)]  # 382 MB each
+    for gf in gfs:
+        gf._destroy()
+    L = c2q.Lattice(32, 64)  # 201 MB a field, as much staging
+    with _Reserve(300 << 20):
+        src = c2q.host.generate_source(L.seo, "z2", 80)
+        f = c2q.Spinorfield_eo(b, L, src)
+        assert np.array_equal(f.dump(), src)
+        f._destroy()
+    assert a.trim() == 0
+    a.close()
+    b.close()
+
+
+def test_a_failed_buffer_leaves_none():
+    """A staging buffer that found no memory: the call fails, a later smaller one works."""
+    import cl2qcd_b200 as c2q
+    s = c2q.System(0)
+    L, l = c2q.Lattice(24, 48), c2q.Lattice(8, 8)  # a full field of 24^3x48: 127 MB
+    small = c2q.host.generate_source(l.seo, "z2", 81)
+    g = c2q.Spinorfield_eo(s, l, small)
+    e, o = c2q.Spinorfield_eo(s, L), c2q.Spinorfield_eo(s, L)
+    s.trim()  # nothing unused is left in the device's pool
+    with _Reserve(64 << 20):
+        with pytest.raises(c2q._lib.C2QError):
+            c2q.host.convert_to_eoprec(e, o, np.zeros((L.vol, 24)))
+        h = c2q.Spinorfield_eo(s, l, small)
+        assert np.array_equal(h.dump(), g.dump())
+    s.close()
+
+
+def test_what_is_kept():
+    """Blocks of a gauge field are kept unless another context has read it; trim gives them back."""
+    import cl2qcd_b200 as c2q
+    a, b = c2q.System(0), c2q.System(0)
+    L = c2q.Lattice(8, 8)
+    g = c2q.host.generate_gaugefield(L, 0.3, 82)
+    src = c2q.host.generate_source(L.seo, "z2", 82)
+    for prec in (64, 16):
+        for reader in (a, b):
+            gf = c2q.Gaugefield(a, L, g)
+            out, inp = c2q.Spinorfield_eo(reader, L, precision=prec), c2q.Spinorfield_eo(reader, L, src, precision=prec)
+            c2q.host.dslash(out, gf, inp, c2q.host.ODD, 0.15)
+            n = a.lib.c2q_gauge_device_bytes(gf.h)
+            gf._destroy()
+            assert a.trim() == (n if reader is a else 0)
+            assert a.trim() == 0 and b.trim() == 0
+    b.close()
+    a.close()
+
+
+def test_server_keeps_no_scratch():
+    """A registered gauge field takes the memory that the budget counts for it, and staging."""
+    import torch
+    import cl2qcd_b200 as c2q
+    L = c2q.Lattice(16, 32)
+    g = c2q.host.generate_gaugefield(L, 0.3, 83)  # 75 MB as uploaded
+    server = c2q.host.Server(0, slots=1, precision=16)
+    free = torch.cuda.mem_get_info()[0]
+    server.add_gauge(1, L, g)
+    used = free - torch.cuda.mem_get_info()[0]
+    counted = server.stats()["gauge_bytes"]
+    server.close()
+    # staging of the upload, and each allocation in whole pages of 2 MiB
+    assert used <= counted + g.nbytes + (32 << 20), (used, counted)
