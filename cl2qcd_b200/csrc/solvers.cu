@@ -739,7 +739,11 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
     // division flag of all right-hand sides into a pinned ring slot and
     // records an event; the host reads iteration k-1 while iteration k runs
     // and applies its decisions after iteration k.
+    // (A cooperative launch hands its last judgements over itself: the ring may still
+    // receive an older iteration's.)
     std::vector<int> hist[4], act;
+    double judged[PK_MAX_RHS];
+    int bad[PK_MAX_RHS];  // SolverScalars::flag
     int iter = 0;
     // Small lattices: the iterations up to the next decision in one launch
     int whole_most = 0;
@@ -795,14 +799,12 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
             if (!rc) rc = pcg_collect(ctx, C, &R);
             if (rc) return rc;
             iter += R.iters - 1;  // the last iteration done
-            hist[(iter + 3) % 4] = act;
             for (int i = 0; i < C.n; ++i) {
                 RhsState& s = S[act[i]];
                 s.sweeps += per_apply * R.iters;
-                s.maxrr       = R.maxrr[i];
-                double* slot  = ctx->batch_ring + (size_t)((iter + 3) % 4) * PK_MAX_RHS * 4 + 4 * act[i];
-                slot[0]       = R.judged[i];
-                memcpy(slot + 3, &R.flag[i], sizeof(int));
+                s.maxrr        = R.maxrr[i];
+                judged[act[i]] = R.judged[i];
+                bad[act[i]]    = R.flag[i];
             }
         } else if (graphs && iter > 0) {
             if (graph.set != act) {
@@ -837,16 +839,21 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
             if (rc) return rc;
         }
         if (iter == 0) continue;
-        if (!whole) C2Q_CUDA(ctx, cudaEventSynchronize(ctx->ring_ev[(iter - 1) % 4]));
-        const double* prev = ctx->batch_ring + (size_t)((iter - 1) % 4) * PK_MAX_RHS * 4;
-        for (int k : hist[(iter - 1) % 4]) {
+        const std::vector<int>& due = whole ? act : hist[(iter - 1) % 4];
+        if (!whole) {
+            C2Q_CUDA(ctx, cudaEventSynchronize(ctx->ring_ev[(iter - 1) % 4]));
+            const double* prev = ctx->batch_ring + (size_t)((iter - 1) % 4) * PK_MAX_RHS * 4;
+            for (int k : due) {
+                judged[k] = prev[4 * k];
+                memcpy(&bad[k], prev + 4 * k + 3, sizeof(int));  // the flag follows resid and aux[2]
+            }
+        }
+        for (int k : due) {
             RhsState& s = S[k];
             if (!s.active || iter - 1 <= s.skip_upto) continue;
-            const double resid = prev[4 * k];
-            int bad            = 0;
-            memcpy(&bad, prev + 4 * k + 3, sizeof(int));  // SolverScalars::flag follows resid and aux[2]
-            s.resid = resid;
-            if (resid != resid || bad) {
+            const double resid = judged[k];
+            s.resid            = resid;
+            if (resid != resid || bad[k]) {
                 s.status = C2Q_SOLVER_STUCK;
                 s.iters  = iter;
                 s.active = false;

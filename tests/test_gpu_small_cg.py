@@ -52,6 +52,45 @@ def test_mixed_iterations_bitwise(port, system, O, ns, nt, precision, rec12, act
         assert np.linalg.norm(r - srcs[k]) / np.linalg.norm(srcs[k]) <= 1.5e-10
 
 
+@pytest.mark.parametrize("precision", [16, 32])
+def test_batch_that_shrinks_into_one_launch(system, precision):
+    """41 tiles a right-hand side, 12 of them: too many for one wave until some have converged
+    (they start at solutions of different quality).  Bitwise the per-launch iterates."""
+    import cl2qcd_b200 as c2q
+    L = c2q.Lattice(12, 12, 1.0, 0.0)
+    gf = c2q.Gaugefield(system, L, c2q.host.generate_gaugefield(L, 0.3, 14))
+    add = c2q.AdditionalParameters(0.14, 2 * 0.14 * 0.05)
+    A = c2q.host.QplusQminus_eo()
+
+    def params(tol):
+        return c2q.SolverParameters(solver="cg", prec=0.0, rel_tol=tol, cgmax=5000, precision=precision,
+                                    use_rec12=True)
+
+    bs = [c2q.Spinorfield_eo(system, L, c2q.host.generate_source(L.seo, "gaussian", 90 + k)) for k in range(12)]
+    start = []
+    for k, b in enumerate(bs):
+        x = c2q.Spinorfield_eo(system, L)
+        if k:
+            c2q.host.cg(x, A, gf, b, params(10.0 ** (-0.75 * k)), add)
+        start.append(x.dump())
+    out = []
+    for per_launch in (0, 1):
+        xs = [c2q.Spinorfield_eo(system, L, s) for s in start]
+        reps = []
+        system.lib.c2q_ctx_profile(system.h, per_launch)
+        try:
+            c2q.host.cg_multi(xs, A, gf, bs, params(1e-10), add, reps)
+        finally:
+            system.lib.c2q_ctx_profile(system.h, 0)
+        out.append(([x.dump() for x in xs], reps))
+    its = [r["iterations"] for r in out[0][1]]
+    assert len(set(its)) > 4 and max(r["true_resid_rel"] for r in out[0][1]) <= 1e-10
+    for k in range(12):
+        assert its[k] == out[1][1][k]["iterations"]
+        assert out[0][1][k]["reliable_updates"] == out[1][1][k]["reliable_updates"]
+        assert np.array_equal(out[0][0][k], out[1][0][k])
+
+
 @pytest.mark.parametrize("ns,nt", LATTICES + [(6, 10)])
 @pytest.mark.parametrize("rec12,action", [(False, "twistedmass"), (True, "wilson")])
 @pytest.mark.parametrize("mode", ["rel_tol", "refresh", "prec"])
