@@ -786,7 +786,9 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
             // A right-hand side alone: whatever ended the iterations, its increment
             // goes into x and the true residual is due, so both are queued behind them
             // without asking.  The update that is expected to be the last takes the
-            // links as uploaded, as below: its residual has no room above thr.
+            // links as uploaded, as below: its residual has no room above thr.  (Where
+            // the residual passed both levels in one step the guess is wrong, and the
+            // true residual is computed again below.)
             const int k0 = act[0];
             spec         = C.n == 1;
             if (!rc && spec) {
@@ -867,15 +869,13 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
                 // reliable update in FP64 after iteration `iter`
                 // (an update expected to be the last one uses the uploaded links;
                 // one that converges unexpectedly on 12-real links is confirmed on them)
-                const int gk_upd = spec ? gk_spec : resid < s.thr ? G64 : gk64;
-                if (spec) {
+                const int gk_upd = resid < s.thr ? G64 : gk64;
+                if (!spec) rc = take_out(k, fused ? nullptr : dsc + k);
+                if (spec && gk_spec == gk_upd)
                     s.r2 = r2_spec;
-                } else {
-                    rc = take_out(k, fused ? nullptr : dsc + k);
-                    if (!rc)
-                        rc = true_residual(ctx, op, g, x[k], b[k], kappa, mubar, action, r64, a64, b64, &s.r2,
-                                           &s.sweeps, gk_upd);
-                }
+                else if (!rc)
+                    rc = true_residual(ctx, op, g, x[k], b[k], kappa, mubar, action, r64, a64, b64, &s.r2, &s.sweeps,
+                                       gk_upd);
                 if (!rc && gk_upd != G64 && s.r2 < s.thr)
                     rc = true_residual(ctx, op, g, x[k], b[k], kappa, mubar, action, r64, a64, b64, &s.r2, &s.sweeps,
                                        G64);

@@ -52,6 +52,32 @@ def test_mixed_iterations_bitwise(port, system, O, ns, nt, precision, rec12, act
         assert np.linalg.norm(r - srcs[k]) / np.linalg.norm(srcs[k]) <= 1.5e-10
 
 
+def test_links_of_the_update_near_the_threshold(system):
+    """The update's level and the threshold passed in one step: the update takes the links that the
+    per-launch path takes.  Row 2 of the links is off by what still counts as SU(3), so that 12- and
+    18-real residuals differ; at this kappa the residual rises between steps, so that some updates
+    end above the threshold and the solve goes on from their residual.  Bitwise the same."""
+    import cl2qcd_b200 as c2q
+    L = c2q.Lattice(8, 8, 1.0, 0.0)
+    g = c2q.host.generate_gaugefield(L, 0.3, 15).reshape(-1, 18).copy()
+    g[:, 12:] += 4e-14 * np.random.default_rng(5).uniform(-1, 1, (len(g), 6))
+    gf = c2q.Gaugefield(system, L, g)
+    add = c2q.AdditionalParameters(0.25, 2 * 0.25 * 0.0005)
+    src = c2q.host.generate_source(L.seo, "gaussian", 52)
+    updates = set()
+    for tol in np.geomspace(0.3, 1e-4, 200):
+        # the update's level, counted from |r| = |b| at the start, lies just above the threshold
+        P = c2q.SolverParameters(solver="cg", prec=0.0, rel_tol=tol, cgmax=20000, precision=16, use_rec12=True,
+                                 reliable_delta=1.01 * tol)
+        xa, ra = _solve(c2q, system, L, gf, [src], P, add)
+        xb, rb = _solve(c2q, system, L, gf, [src], P, add, per_launch=True)
+        assert ra[0]["iterations"] == rb[0]["iterations"]
+        assert ra[0]["reliable_updates"] == rb[0]["reliable_updates"]
+        assert np.array_equal(xa[0], xb[0]), tol
+        updates.add(ra[0]["reliable_updates"])
+    assert len(updates) > 1  # some solves did go on
+
+
 @pytest.mark.parametrize("precision", [16, 32])
 def test_batch_that_shrinks_into_one_launch(system, precision):
     """41 tiles a right-hand side, 12 of them: too many for one wave until some have converged
