@@ -90,6 +90,10 @@ struct c2q_ctx {
     // launch predicate of a device-driven solve (SolverScalars::halt): while set,
     // every reducing BLAS and dslash launch skips its work once *halt_dev != 0
     const int* halt_dev = nullptr;
+    // the cooperative CG iterations: polls of a wait at a grid barrier (0: none of these
+    // launches), and how many launches were given up
+    unsigned barrier_polls = 1u << 22;  // some seconds; a block of a resident grid arrives within microseconds
+    long long barrier_giveups = 0;
     int sm_count  = 0;
     // pinned ring of the batched solvers: 4 slots x 16 right-hand sides x 4 doubles
     double* batch_ring = nullptr;
@@ -341,7 +345,8 @@ struct PcgBatch {
     void* ctl = nullptr;  // pcg_ctl_bytes() of device memory
 };
 struct PcgResult {
-    int iters;  // done; the last one judged the residual of the one before
+    bool gave_up;  // at a barrier: p, rs, xs and the scalars hold no one iteration's state
+    int iters;     // done; the last one judged the residual of the one before
     double judged[MAX_BATCH], maxrr[MAX_BATCH];
     int flag[MAX_BATCH];
 };
@@ -371,6 +376,7 @@ struct Pcg64Solve {
     double thr;
 };
 struct Pcg64Result {
+    bool gave_up;  // at a barrier: x may hold a part of the last update, the rest no one iteration's state
     int iters, stop;
     double judged;
 };

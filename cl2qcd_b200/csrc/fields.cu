@@ -958,6 +958,15 @@ C2Q_EXPORT int c2q_ctx_create(c2q_ctx** out, int device, void* cuda_stream)
     return C2Q_OK;
 }
 
+C2Q_EXPORT int c2q_ctx_set_barrier_polls(c2q_ctx* ctx, unsigned polls)
+{
+    if (!ctx) return C2Q_BAD_ARG;
+    ctx->barrier_polls = polls;
+    return C2Q_OK;
+}
+
+C2Q_EXPORT long long c2q_ctx_barrier_giveups(const c2q_ctx* ctx) { return ctx ? ctx->barrier_giveups : 0; }
+
 C2Q_EXPORT int c2q_ctx_trim(c2q_ctx* ctx, size_t* bytes)
 {
     if (!ctx) return C2Q_BAD_ARG;

@@ -8,11 +8,10 @@ namespace c2q {
 // far.  Writes before it are visible to every block after it (the acquiring
 // load also drops the SM's L1 lines); data that the kernel changes must not be
 // read through the non-coherent path.  Returns false once a wait has run out of
-// polls (some seconds; a block of a resident grid arrives within microseconds)
-// or another block's wait has: the error word is then set and every block
-// leaves.
-constexpr unsigned GRIDBAR_POLLS = 1u << 22;
-__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned* error, unsigned target, int* ok)
+// `polls` or another block's wait has: the error word is then set and every block
+// leaves, whatever it had got to; the fields hold any mixture of finished steps.
+__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned* error, unsigned target, unsigned polls,
+                                             int* ok)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -22,7 +21,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned* error,
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
             if (seen >= target) break;
-            if (++n >= GRIDBAR_POLLS || ((n & 1023u) == 0 && *(volatile unsigned*)error)) {
+            if (++n >= polls || ((n & 1023u) == 0 && *(volatile unsigned*)error)) {
                 atomicExch(error, 1u);
                 good = 0;
                 break;

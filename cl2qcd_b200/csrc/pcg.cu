@@ -23,7 +23,8 @@ static int pcg_resident(c2q_ctx* ctx, int* blocks)
 int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* most)
 {
     *most = 0;
-    if (ctx->profiling) return C2Q_OK;  // per-launch timing wants the sweeps as launches of their own
+    // (per-launch timing wants the sweeps as launches of their own)
+    if (ctx->profiling || !ctx->barrier_polls) return C2Q_OK;
     int blocks = 0;
     const int rc = prec == 16 ? (gkind_is_r12(gkind) ? pcg_resident<16, 6>(ctx, &blocks) : pcg_resident<16, 9>(ctx, &blocks))
                               : (gkind_is_r12(gkind) ? pcg_resident<32, 6>(ctx, &blocks) : pcg_resident<32, 9>(ctx, &blocks));
@@ -84,6 +85,7 @@ int pcg_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B)
     prm.delta  = B.delta;
     prm.first  = B.first;
     prm.iters  = B.iters;
+    prm.polls  = ctx->barrier_polls;
     int rc     = ensure_partials(ctx, (size_t)prm.ntiles * PK_WARPS * B.n);
     if (rc) return rc;
     prm.partials = ctx->partials;
@@ -102,7 +104,11 @@ int pcg_collect(c2q_ctx* ctx, const PcgBatch& B, PcgResult* out)
     C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     PcgCtl c;
     memcpy(&c, ctx->host_pinned + PCG_PINNED, sizeof c);
-    if (c.error || c.iters < 1) return fail(ctx, C2Q_CUDA_ERROR, "cooperative CG: a grid barrier gave up");
+    out->gave_up = c.error || c.iters < 1;
+    if (out->gave_up) {
+        ++ctx->barrier_giveups;
+        return C2Q_OK;
+    }
     out->iters = c.iters;
     for (int r = 0; r < B.n; ++r) {
         out->judged[r] = c.judged[r];

@@ -247,9 +247,9 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
     const int gk = gk64_for(g, P->use_rec12);
     int sweeps   = 0;
     SolveClock clock(ctx);
-    const bool small = pcg64_applies(ctx, op, g);
+    bool small = pcg64_applies(ctx, op, g);
     // Q+Q- with the vector updates in its sweeps
-    const bool fused = !small && op == C2Q_OP_QPLUSQMINUS_EO && adjoint_weights(g);
+    const bool fused = op == C2Q_OP_QPLUSQMINUS_EO && adjoint_weights(g);
     double x2 = 0;
     rc        = norm2(ctx, x, &x2);
     if (rc) return rc;
@@ -290,6 +290,7 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
     int iter = 0, status = C2Q_DID_NOT_SOLVE;
     double resid = std::numeric_limits<double>::quiet_NaN();
     bool force_refresh = false;
+    int skip_upto      = -1;     // iterations whose residual is not judged (rel_tol)
     double r2_confirmed = -1.0;  // true residual of the returned solution, when already computed
     if (small) {
         // Small lattices: everything between two refreshes in one launch.  With
@@ -298,7 +299,6 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
         // resid_check_every-th, at once.
         const bool lag = P->rel_tol > 0;
         const int end  = std::max(P->cgmax, P->min_iter);
-        int skip_upto  = -1;
         while (iter < end) {
             Pcg64Solve S{x, rn, p, t1, t2, kappa, mubar, action};
             if (iter % P->iter_refresh == 0 || force_refresh) {
@@ -317,6 +317,13 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
             Pcg64Result R;
             rc = pcg64_run(ctx, g, gk, S, &R);
             if (rc) return rc;
+            if (R.gave_up) {
+                // whatever part of x was updated, the per-launch iterations go on from its true residual
+                small         = false;
+                force_refresh = true;
+                skip_upto     = iter - 1;
+                break;
+            }
             sweeps += 4 * R.iters;
             iter += R.iters - 1;  // the last iteration done
             if (R.stop || R.judged == R.judged) resid = R.judged;
@@ -342,12 +349,12 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
             }
             ++iter;
         }
-    } else if (P->rel_tol > 0) {
+    }
+    if (!small && P->rel_tol > 0) {
         // True-residual target: residual monitored every iteration through the
         // pinned ring (no host round trip per iteration); a converged iterated
         // residual is confirmed by an FP64 true residual, else CG restarts from it.
         ResidRing ring(ctx);
-        int skip_upto = -1;
         // With use_graph the iteration body between refreshes (p = rn + beta p,
         // v = A p with (p, v) -> alpha, the x / rn update) replays as one captured
         // CUDA graph: small lattices are bound by launch latency.  It is captured
@@ -362,7 +369,7 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
         } gexec;
         long long gkernels = 0;
         int gsweeps        = 0;
-        for (iter = 0; iter < P->cgmax || iter < P->min_iter; iter++) {
+        for (; iter < P->cgmax || iter < P->min_iter; iter++) {
             if (iter % P->iter_refresh == 0 || force_refresh) {
                 force_refresh = false;
                 rc            = refresh();
@@ -419,8 +426,8 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
                 skip_upto     = iter;
             }
         }
-    } else {
-        for (iter = 0; iter < P->cgmax || iter < P->min_iter; iter++) {
+    } else if (!small) {
+        for (; iter < P->cgmax || iter < P->min_iter; iter++) {
             if (iter % P->iter_refresh == 0 || force_refresh) {
                 force_refresh = false;
                 rc            = refresh();
@@ -545,10 +552,13 @@ int accumulate(c2q_ctx* ctx, c2q_spinor_eo* x, c2q_spinor_eo* xs, const c2q_spin
     return C2Q_OK;
 }
 
-// A right-hand side's scalars at the start (zeroed before): omega = (r, r).
+// A right-hand side's scalars at the start: omega = (r, r), the rest zero.
 __global__ void mixed_start_kernel(SolverScalars* s, double r2)
 {
-    if (threadIdx.x == 0) s->omega[0] = r2;
+    if (threadIdx.x != 0) return;
+    SolverScalars z{};
+    z.omega[0] = r2;
+    *s         = z;
 }
 
 // A reliable update's scalars: beta rescaled to the true residual r2 (the
@@ -649,8 +659,20 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
         return use_tg ? tg_accumulate(ctx, g, x[k], xs[k], p[k], sc) : accumulate<PB>(ctx, x[k], xs[k], p[k], sc);
     };
 
-    // ---- initial residuals
     RhsState S[PK_MAX_RHS];
+    // the iteration starts at the residual r, |r|^2 = S[k].r2: p = r, beta = 0
+    auto start = [&](int k, const c2q_spinor_eo* r) -> int {
+        int e = to_inner(rs[k], r);
+        if (!e) e = launch_convert(ctx, p[k], rs[k]);
+        if (e) return e;
+        mixed_start_kernel<<<1, 32, 0, ctx->stream>>>(dsc + k, S[k].r2);
+        ctx->launches++;
+        C2Q_CUDA(ctx, cudaGetLastError());
+        S[k].maxrr = std::sqrt(S[k].r2);
+        return C2Q_OK;
+    };
+
+    // ---- initial residuals
     for (int k = 0; k < n; ++k) {
         RhsState& s = S[k];
         rc          = saxpy_norm(ctx, r64, Cx{0, 0}, b[k], b[k], FIN_STORE_RESULT, &s.b2);
@@ -659,13 +681,11 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
         double x2 = 0;
         rc        = norm2(ctx, x[k], &x2);
         if (rc) return rc;
-        if (x2 == 0.0) {  // r = b - A 0 = b
-            rc   = to_inner(rs[k], b[k]);
+        const bool zero_x = x2 == 0.0;  // r = b - A 0 = b
+        if (zero_x)
             s.r2 = s.b2;
-        } else {
+        else
             rc = true_residual(ctx, op, g, x[k], b[k], kappa, mubar, action, r64, a64, b64, &s.r2, &s.sweeps, G64);
-            if (!rc) rc = to_inner(rs[k], r64);
-        }
         if (rc) return rc;
         s.resid = s.r2;
         // r = 0 (a zero source with a zero start): x is exact and alpha would be 0/0
@@ -675,12 +695,8 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
             continue;
         }
         rc = c2q_spinor_eo_zero(xs[k]);
-        if (!rc) rc = launch_convert(ctx, p[k], rs[k]);
+        if (!rc) rc = start(k, zero_x ? b[k] : r64);
         if (rc) return rc;
-        mixed_start_kernel<<<1, 32, 0, ctx->stream>>>(dsc + k, s.r2);
-        ctx->launches++;
-        C2Q_CUDA(ctx, cudaGetLastError());
-        s.maxrr  = std::sqrt(s.r2);
         s.active = true;
     }
 
@@ -690,7 +706,7 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
     // and the residual update in the last one; otherwise x_s += alpha p is
     // deferred to the next mix_p or to the reliable-update accumulation
     const bool fused    = op == C2Q_OP_QPLUSQMINUS_EO;
-    const bool graphs   = P->use_graph && !ctx->profiling;
+    bool graphs         = P->use_graph && !ctx->profiling;
     BatchGraph graph;
     auto body = [&](const std::vector<int>& A, bool with_p) -> int {
         const int m = (int)A.size();
@@ -800,6 +816,24 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
             }
             if (!rc) rc = pcg_collect(ctx, C, &R);
             if (rc) return rc;
+            if (R.gave_up) {
+                // The per-launch iterations (eager: no shape of theirs has been sized) start
+                // again from the true residuals of what the solutions have, whatever part of
+                // an update that is.
+                whole_most = 0;
+                graphs     = false;
+                for (int k : act) {
+                    RhsState& s = S[k];
+                    rc          = take_out(k, nullptr);
+                    if (!rc)
+                        rc = true_residual(ctx, op, g, x[k], b[k], kappa, mubar, action, r64, a64, b64, &s.r2, &s.sweeps,
+                                           G64);
+                    if (!rc) rc = start(k, r64);
+                    if (rc) return rc;
+                    s.skip_upto = iter;
+                }
+                continue;
+            }
             iter += R.iters - 1;  // the last iteration done
             for (int i = 0; i < C.n; ++i) {
                 RhsState& s = S[act[i]];

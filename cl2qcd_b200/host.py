@@ -102,6 +102,15 @@ class System:
         """Pin the launch choice of the reduced-precision sweeps (-1: the autotuner's)."""
         _check(self.lib.c2q_ctx_set_sweep_choice(self.h, choice), self.h, self.lib)
 
+    def set_barrier_polls(self, polls: int):
+        """Bound of a wait in the cooperative CG launches of small lattices (0: ordinary launches only)."""
+        _check(self.lib.c2q_ctx_set_barrier_polls(self.h, polls), self.h, self.lib)
+
+    @property
+    def barrier_giveups(self) -> int:
+        """Cooperative launches given up at a barrier; their solves went on with ordinary launches."""
+        return self.lib.c2q_ctx_barrier_giveups(self.h)
+
     def tune_report(self) -> str:
         """The launch configurations the autotuner chose, one line per launch shape."""
         n = self.lib.c2q_ctx_tune_report(self.h, None, 0)

@@ -141,6 +141,39 @@ def test_fp64_iterations(port, system, O, ns, nt, rec12, action, mode):
     assert rel_l2(xa[0], xb[0]) <= 1e-8
 
 
+@pytest.mark.parametrize("precision,mode", [(64, "rel_tol"), (64, "prec"), (64, "graph"), (32, "one"), (16, "one"),
+                                            (16, "batch"), (16, "graph")])
+def test_a_barrier_that_gives_up(port, O, precision, mode):
+    """Waits of one poll run out at once: the launch is given up and the solve goes on without it.
+    The context works as before afterwards."""
+    import cl2qcd_b200 as c2q
+    system = c2q.System(0)
+    port.set_lattice(8, 16, 1.0, 0.0)
+    L = c2q.Lattice(8, 16, 1.0, 0.0)
+    g = c2q.host.generate_gaugefield(L, 0.3, 16)
+    gf = c2q.Gaugefield(system, L, g)
+    kappa, mubar = 0.14, 2 * 0.14 * 0.05
+    add = c2q.AdditionalParameters(kappa, mubar)
+    srcs = [c2q.host.generate_source(L.seo, "gaussian", 53 + k) for k in range(5 if mode == "batch" else 1)]
+    kw = dict(prec=1e-20 * float(np.sum(srcs[0] ** 2))) if mode == "prec" else dict(prec=0.0, rel_tol=1e-10)
+    P = c2q.SolverParameters(solver="cg", cgmax=5000, precision=precision, use_rec12=True, use_graph=mode == "graph",
+                             **kw)
+    want, rep = _solve(c2q, system, L, gf, srcs, P, add)
+    assert system.barrier_giveups == 0
+    system.set_barrier_polls(1)
+    xs, reps = _solve(c2q, system, L, gf, srcs, P, add)
+    assert system.barrier_giveups == 1
+    for k, s in enumerate(srcs):
+        r = port.apply(O.OP_QPQM_EO, xs[k], g, kappa, mubar)
+        assert np.linalg.norm(r - s) / np.linalg.norm(s) <= 1.5e-10
+        # one iteration lost and the search direction begun anew; with prec a check interval of 10
+        assert reps[k]["iterations"] <= rep[k]["iterations"] + 10
+    system.set_barrier_polls(1 << 22)
+    again, _ = _solve(c2q, system, L, gf, srcs, P, add)
+    assert all(np.array_equal(a, w) for a, w in zip(again, want)) and system.barrier_giveups == 1
+    system.close()
+
+
 @pytest.mark.parametrize("precision", [64, 32, 16])
 def test_limits_and_nan(system, precision):
     """The iteration limit and a residual that is no number end the solve as before."""
