@@ -23,8 +23,8 @@ static int pcg_resident(c2q_ctx* ctx, int* blocks)
 int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* most)
 {
     *most = 0;
-    // (per-launch timing wants the sweeps as launches of their own)
-    if (ctx->profiling || !ctx->barrier_polls) return C2Q_OK;
+    // (per-launch timing and a pinned sweep choice want the sweeps as launches of their own)
+    if (ctx->profiling || ctx->force_choice >= 0 || !ctx->barrier_polls) return C2Q_OK;
     int blocks = 0;
     const int rc = prec == 16 ? (gkind_is_r12(gkind) ? pcg_resident<16, 6>(ctx, &blocks) : pcg_resident<16, 9>(ctx, &blocks))
                               : (gkind_is_r12(gkind) ? pcg_resident<32, 6>(ctx, &blocks) : pcg_resident<32, 9>(ctx, &blocks));

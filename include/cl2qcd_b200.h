@@ -299,9 +299,9 @@ C2Q_EXPORT int c2q_ctx_set_autotune(c2q_ctx* ctx, int enable);
  * launch configuration (choice & 1) with one block per tile (choice >> 1 = 0)
  * or a grid-stride grid (1); 4 = two right-hand sides per thread, for FP16
  * batches of two or more in the temporal gauge (elsewhere choice 0); -1 = the
- * autotuner decides (default).  Every choice gives bitwise the same results.  The
- * mixed-precision CG on QplusQminus_eo of small lattices runs whole iterations in
- * one cooperative launch (bitwise the same too), which has no choice. */
+ * autotuner decides (default).  Every choice gives bitwise the same results, and so do
+ * the cooperative launches of small lattices' mixed-precision CG, which are left out
+ * while a choice is pinned. */
 C2Q_EXPORT int c2q_ctx_set_sweep_choice(c2q_ctx* ctx, int choice);
 C2Q_EXPORT int c2q_ctx_tune_report(const c2q_ctx* ctx, char* buf, int len);
 /* (no counterpart in the reference) On small lattices the CG on QplusQminus_eo runs many

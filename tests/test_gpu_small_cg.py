@@ -174,6 +174,28 @@ def test_a_barrier_that_gives_up(port, O, precision, mode):
     system.close()
 
 
+@pytest.mark.parametrize("choice,n", [(0, 1), (3, 1), (4, 3)])
+def test_a_pinned_sweep_choice_is_run(system, choice, n):
+    """While a choice is pinned the sweeps are launches of their own, with that choice: at least the
+    four of an iteration and its p update, and bitwise the cooperative launch's solutions."""
+    import cl2qcd_b200 as c2q
+    L = c2q.Lattice(6, 12, 1.0, 0.0)
+    gf = c2q.Gaugefield(system, L, c2q.host.generate_gaugefield(L, 0.3, 17))
+    add = c2q.AdditionalParameters(0.14, 2 * 0.14 * 0.05)
+    srcs = [c2q.host.generate_source(L.seo, "gaussian", 56 + k) for k in range(n)]
+    P = c2q.SolverParameters(solver="cg", prec=0.0, rel_tol=1e-10, cgmax=5000, precision=16, use_rec12=True)
+    want, rep = _solve(c2q, system, L, gf, srcs, P, add)
+    system.set_sweep_choice(choice)
+    try:
+        before = system.launch_count
+        xs, reps = _solve(c2q, system, L, gf, srcs, P, add)
+        launches = system.launch_count - before
+    finally:
+        system.set_sweep_choice(-1)
+    assert launches >= 5 * max(r["iterations"] for r in reps)
+    assert all(np.array_equal(a, b) for a, b in zip(xs, want))
+
+
 @pytest.mark.parametrize("precision", [64, 32, 16])
 def test_limits_and_nan(system, precision):
     """The iteration limit and a residual that is no number end the solve as before."""
