@@ -23,7 +23,8 @@ static void parallel_copy(char* dst, const char* src, size_t n)
 {
     constexpr size_t PIECE = (size_t)256 << 10;
     const long long pieces = (long long)((n + PIECE - 1) / PIECE);
-    const int threads      = std::max(1, std::min(8, omp_get_num_procs()));
+    // eight fill PCIe; fewer where the caller's OpenMP setting or the process's cores say so
+    const int threads = std::max(1, std::min({8, omp_get_num_procs(), omp_get_max_threads()}));
 #pragma omp parallel for num_threads(threads) schedule(static)
     for (long long k = 0; k < pieces; ++k) {
         const size_t at = (size_t)k * PIECE;

@@ -1,8 +1,14 @@
 """GPU: transfers of pageable and pinned host arrays (hostcopy.cu) around the chunk and
 ring sizes (4 MiB chunks, a ring of four; below two chunks the plain copy): what comes
 back is what went in, bit for bit."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
+
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +42,24 @@ def test_round_trip(system, ns, nt, pinned):
     assert np.array_equal(c2q.Gaugefield(system, L, u).download(), u)
     m = host((4 * L.vol, 8))
     assert np.array_equal(c2q.host.Gaugemomenta(system, L, m).download(), m)
+
+
+@pytest.mark.parametrize("threads", [1, 3])
+def test_omp_num_threads(lib, threads):
+    """The copies take no more threads than OMP_NUM_THREADS allows (a launcher sets it to 1 where
+    every GPU has its own process)."""
+    code = """
+import os, numpy as np, cl2qcd_b200 as c2q
+s = c2q.System(0)
+L = c2q.Lattice(18, 16)
+f = c2q.Spinorfield_eo(s, L)
+a = np.ones((L.seo, 24))
+n = len(os.listdir("/proc/self/task"))
+f.load(a)
+assert np.array_equal(f.dump(), a)
+print("new threads:", len(os.listdir("/proc/self/task")) - n)
+"""
+    env = dict(os.environ, OMP_NUM_THREADS=str(threads), PYTHONPATH=ROOT)
+    out = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    assert int(out.stdout.split("new threads:")[1]) <= threads - 1
