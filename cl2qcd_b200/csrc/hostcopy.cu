@@ -32,7 +32,8 @@ static void parallel_copy(char* dst, const char* src, size_t n)
     }
 }
 
-// whether the ring serves this copy (and make the ring)
+// whether the ring serves this copy (and make the ring; without pinned memory for it the
+// copy goes through the driver's staging)
 static int use_ring(c2q_ctx* ctx, const void* host, size_t bytes, bool* ring)
 {
     *ring = false;
@@ -45,8 +46,13 @@ static int use_ring(c2q_ctx* ctx, const void* host, size_t bytes, bool* ring)
     }
     if (a.type != cudaMemoryTypeUnregistered) return C2Q_OK;  // pinned: the engine takes it as it is
     if (!ctx->hc_ring) {
-        C2Q_CUDA(ctx, cudaMallocHost(&ctx->hc_ring, HC_RING * HC_CHUNK));
-        for (auto& ev : ctx->hc_ev) C2Q_CUDA(ctx, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        for (auto& ev : ctx->hc_ev)
+            if (!ev) C2Q_CUDA(ctx, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        if (cudaMallocHost(&ctx->hc_ring, HC_RING * HC_CHUNK) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->hc_ring = nullptr;
+            return C2Q_OK;
+        }
     }
     *ring = true;
     return C2Q_OK;
