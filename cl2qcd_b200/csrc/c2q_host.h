@@ -350,13 +350,38 @@ struct PcgResult {
     double judged[MAX_BATCH], maxrr[MAX_BATCH];
     int flag[MAX_BATCH];
 };
-// *most: the largest batch that takes these iterations on a lattice of geometry g
-// -- every tile of every right-hand side needs a resident block of its own (one
+// *tiles: the blocks a right-hand side takes on a lattice of geometry g; *room: the blocks
+// of the device, 0 where these iterations are not to be taken.  A batch takes them if
+// every tile of every right-hand side has a resident block of its own (one
 // wave).  With more, a phase runs a second, partly empty wave between two
 // barriers and the ordinary launches are as fast or faster: FP16, per iteration
 // with its share of the reliable updates, 16^3x32 (256 tiles) 53 us against 69 us,
 // 20^3x40 (625 tiles) 110 against 104, four sources at 16^3x32 165 against 144.
-int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* most);
+int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* tiles, int* room);
+// Blocks of cooperative CG launches in flight on a device, all contexts together.  The
+// hardware starts such a launch only once all its blocks have room, so grids that do
+// not fit side by side run one after the other, and whatever is queued behind them
+// waits: two 16^3x32 solves at a time took 20.7 ms each against 17.8 ms with launches of
+// their own, a light request beside three of them up to 33 ms against 13 ms.  `most`
+// blocks fit with what is in flight, or (most 0) they are counted without a test.
+bool coop_enter(int device, int blocks, int most);
+void coop_leave(int device, int blocks);
+struct CoopRoom {  // a launch's share, given back when its results are in
+    int device, blocks;
+    bool got;
+    CoopRoom(int device, int blocks, int most)
+        : device(device), blocks(blocks), got(blocks > 0 && coop_enter(device, blocks, most))
+    {
+    }
+    ~CoopRoom() { leave(); }
+    void leave()
+    {
+        if (got) coop_leave(device, blocks);
+        got = false;
+    }
+    CoopRoom(const CoopRoom&)            = delete;
+    CoopRoom& operator=(const CoopRoom&) = delete;
+};
 size_t pcg_ctl_bytes();
 // launch without waiting; collect waits for the stream, and so for what was queued since
 int pcg_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B);

@@ -1,5 +1,6 @@
 // pcg.cu -- host side of pcg.cuh: the cooperative launch that runs the
 // iterations of the mixed-precision CG on small lattices.
+#include <atomic>
 #include <cstring>
 
 #include "c2q_host.h"
@@ -20,17 +21,28 @@ static int pcg_resident(c2q_ctx* ctx, int* blocks)
     return C2Q_OK;
 }
 
-int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* most)
+static std::atomic<int> coop_blocks[64];
+
+bool coop_enter(int device, int blocks, int most)
 {
-    *most = 0;
+    std::atomic<int>& in_flight = coop_blocks[device & 63];
+    int now                     = in_flight.load(std::memory_order_relaxed);
+    do {
+        if (most && now + blocks > most) return false;
+    } while (!in_flight.compare_exchange_weak(now, now + blocks, std::memory_order_relaxed));
+    return true;
+}
+
+void coop_leave(int device, int blocks) { coop_blocks[device & 63].fetch_sub(blocks, std::memory_order_relaxed); }
+
+int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* tiles, int* room)
+{
+    *tiles = (g.seo / 2 + PK_THREADS - 1) / PK_THREADS;
+    *room  = 0;
     // (per-launch timing and a pinned sweep choice want the sweeps as launches of their own)
     if (ctx->profiling || ctx->force_choice >= 0 || !ctx->barrier_polls) return C2Q_OK;
-    int blocks = 0;
-    const int rc = prec == 16 ? (gkind_is_r12(gkind) ? pcg_resident<16, 6>(ctx, &blocks) : pcg_resident<16, 9>(ctx, &blocks))
-                              : (gkind_is_r12(gkind) ? pcg_resident<32, 6>(ctx, &blocks) : pcg_resident<32, 9>(ctx, &blocks));
-    if (rc) return rc;
-    *most = blocks / ((g.seo / 2 + PK_THREADS - 1) / PK_THREADS);
-    return C2Q_OK;
+    return prec == 16 ? (gkind_is_r12(gkind) ? pcg_resident<16, 6>(ctx, room) : pcg_resident<16, 9>(ctx, room))
+                      : (gkind_is_r12(gkind) ? pcg_resident<32, 6>(ctx, room) : pcg_resident<32, 9>(ctx, room));
 }
 
 // where the control block lands in the context's pinned buffer (read_scalars uses its head)

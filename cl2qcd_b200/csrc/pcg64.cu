@@ -290,15 +290,17 @@ __global__ void __launch_bounds__(THREADS64, 2) pcg64_kernel(const Params64 prm)
     }
 }
 
-template <int NL>
-int go64(c2q_ctx* ctx, Params64& prm)
+int blocks64(c2q_ctx* ctx, const void* kern, int ntiles, int* blocks)
 {
-    const void* kern = (const void*)pcg64_kernel<NL>;
     int per_sm = 0, sms = 0;
     C2Q_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS64, 0));
     C2Q_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    int blocks = prm.ntiles < per_sm * sms ? prm.ntiles : per_sm * sms;
-    if (blocks < 1) return fail(ctx, C2Q_CUDA_ERROR, "cooperative CG: no resident block");
+    *blocks = ntiles < per_sm * sms ? ntiles : per_sm * sms;
+    return *blocks < 1 ? fail(ctx, C2Q_CUDA_ERROR, "cooperative CG: no resident block") : C2Q_OK;
+}
+
+int go64(c2q_ctx* ctx, const void* kern, int blocks, Params64& prm)
+{
     C2Q_CUDA(ctx, cudaMemsetAsync(prm.ctl, 0, sizeof(Ctl64), ctx->stream));
     void* args[] = {&prm};
     C2Q_CUDA(ctx, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(THREADS64), args, 0, ctx->stream));
@@ -361,7 +363,14 @@ int pcg64_run(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const Pcg64Solve& S, 
     if (rc) return rc;
     prm.partials = ctx->partials;
     prm.ctl      = reinterpret_cast<Ctl64*>(ctx->partials + prm.ntiles + (prm.ntiles & 1));
-    rc           = gkind_is_r12(gkind) ? go64<6>(ctx, prm) : go64<9>(ctx, prm);
+    const void* kern = gkind_is_r12(gkind) ? (const void*)pcg64_kernel<6> : (const void*)pcg64_kernel<9>;
+    int blocks       = 0;
+    rc               = blocks64(ctx, kern, prm.ntiles, &blocks);
+    if (rc) return rc;
+    // counted, but not tested for room: these iterates differ from the ordinary launches'
+    // by rounding, and results do not depend on what else runs
+    const CoopRoom share(ctx->device, blocks, 0);
+    rc = go64(ctx, kern, blocks, prm);
     if (!rc) rc = pinned_copy(ctx, ctx->host_pinned_dev, 0, prm.ctl, 0, sizeof(Ctl64));
     if (rc) return rc;
     C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -706,7 +706,7 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
     // and the residual update in the last one; otherwise x_s += alpha p is
     // deferred to the next mix_p or to the reliable-update accumulation
     const bool fused    = op == C2Q_OP_QPLUSQMINUS_EO;
-    bool graphs         = P->use_graph && !ctx->profiling;
+    const bool graphs   = P->use_graph && !ctx->profiling;
     BatchGraph graph;
     auto body = [&](const std::vector<int>& A, bool with_p) -> int {
         const int m = (int)A.size();
@@ -761,17 +761,31 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
     double judged[PK_MAX_RHS];
     int bad[PK_MAX_RHS];  // SolverScalars::flag
     int iter = 0;
-    // Small lattices: the iterations up to the next decision in one launch
-    int whole_most = 0;
-    if (use_tg && fused) rc = pcg_capacity(ctx, PB, gk, x[0]->geom, &whole_most);
+    // Small lattices: the iterations up to the next decision in one launch, while its
+    // blocks have room beside other contexts' launches of the kind; the iterations in
+    // between are ordinary ones, bitwise the same
+    int tiles = 0, room = 0;
+    if (use_tg && fused) rc = pcg_capacity(ctx, PB, gk, x[0]->geom, &tiles, &room);
     if (rc) return rc;
+    bool sized  = false;  // an ordinary iteration has run: its launches may be captured
+    int pushed  = -1;     // the last iteration whose residuals went into the ring
+    auto push   = [&](int it) -> int {
+        pushed = it;
+        return ring_push(ctx, it, ctx->batch_ring_dev + (size_t)(it % 4) * PK_MAX_RHS * 4, &dsc[0].resid,
+                         sizeof(SolverScalars), 4 * sizeof(double), n);
+    };
     for (iter = 0; iter < P->cgmax; ++iter) {
         act.clear();
         for (int k = 0; k < n; ++k)
             if (S[k].active) act.push_back(k);
         if (act.empty()) break;
         hist[iter % 4]   = act;
-        const bool whole = (int)act.size() <= whole_most;
+        CoopRoom share(ctx->device, (int)act.size() * tiles <= room ? (int)act.size() * tiles : 0, room);
+        const bool whole = share.got;
+        if (!whole && iter > 0 && pushed != iter - 1) {  // the last iteration was a cooperative launch's
+            rc = push(iter - 1);
+            if (rc) return rc;
+        }
         bool spec        = false;  // the update's residual is there already (r2_spec, on links gk_spec)
         int gk_spec      = G64;
         double r2_spec   = 0;
@@ -815,13 +829,12 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
                                        &S[k0].sweeps, gk_spec);
             }
             if (!rc) rc = pcg_collect(ctx, C, &R);
+            share.leave();
             if (rc) return rc;
             if (R.gave_up) {
-                // The per-launch iterations (eager: no shape of theirs has been sized) start
-                // again from the true residuals of what the solutions have, whatever part of
-                // an update that is.
-                whole_most = 0;
-                graphs     = false;
+                // The ordinary iterations start again from the true residuals of what the
+                // solutions have, whatever part of an update that is.
+                room = 0;
                 for (int k : act) {
                     RhsState& s = S[k];
                     rc          = take_out(k, nullptr);
@@ -835,6 +848,7 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
                 continue;
             }
             iter += R.iters - 1;  // the last iteration done
+            hist[iter % 4] = act;
             for (int i = 0; i < C.n; ++i) {
                 RhsState& s = S[act[i]];
                 s.sweeps += per_apply * R.iters;
@@ -842,7 +856,7 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
                 judged[act[i]] = R.judged[i];
                 bad[act[i]]    = R.flag[i];
             }
-        } else if (graphs && iter > 0) {
+        } else if (graphs && iter > 0 && sized) {
             if (graph.set != act) {
                 graph.reset();
                 cudaGraph_t gr     = nullptr;
@@ -867,11 +881,11 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
         } else {
             rc = body(act, iter > 0);
             if (rc) return rc;
+            sized = true;
         }
         if (!whole) {
             for (int k : act) S[k].sweeps += per_apply;
-            rc = ring_push(ctx, iter, ctx->batch_ring_dev + (size_t)(iter % 4) * PK_MAX_RHS * 4, &dsc[0].resid,
-                           sizeof(SolverScalars), 4 * sizeof(double), n);
+            rc = push(iter);
             if (rc) return rc;
         }
         if (iter == 0) continue;

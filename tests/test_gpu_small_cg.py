@@ -174,6 +174,52 @@ def test_a_barrier_that_gives_up(port, O, precision, mode):
     system.close()
 
 
+def test_solves_side_by_side():
+    """Cooperative grids of several contexts that do not fit side by side: some iterations run as
+    ordinary launches, in between and with graphs, and every solution is bitwise that of a solve
+    with the device to itself."""
+    import threading
+
+    import cl2qcd_b200 as c2q
+    L = c2q.Lattice(12, 12, 1.0, 0.0)  # 41 tiles: seven sources fill two thirds of the device
+    g = c2q.host.generate_gaugefield(L, 0.3, 18)
+    add = c2q.AdditionalParameters(0.15, 2 * 0.15 * 0.01)
+    srcs = [c2q.host.generate_source(L.seo, "gaussian", 57 + k) for k in range(7)]
+
+    def params(graph):
+        return c2q.SolverParameters(solver="cg", prec=0.0, rel_tol=1e-10, cgmax=5000, precision=16, use_rec12=True,
+                                    use_graph=graph)
+
+    alone = c2q.System(0)
+    want, reps = _solve(c2q, alone, L, c2q.Gaugefield(alone, L, g), srcs, params(False), add)
+    cooperative = alone.launch_count
+    bad = []
+
+    def work(i):
+        try:
+            s = c2q.System(0)
+            gf = c2q.Gaugefield(s, L, g)
+            for k in range(8):
+                xs, r = _solve(c2q, s, L, gf, srcs, params(bool((i + k) % 2)), add)
+                assert [q["iterations"] for q in r] == [q["iterations"] for q in reps]
+                assert all(np.array_equal(a, b) for a, b in zip(xs, want))
+            launches[i] = s.launch_count
+            s.close()
+        except Exception as e:
+            bad.append(e)
+
+    launches = [0] * 4
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad, bad
+    # (both kinds of iteration were met: a cooperative solve has few launches)
+    assert max(launches) > 8 * cooperative
+    alone.close()
+
+
 @pytest.mark.parametrize("choice,n", [(0, 1), (3, 1), (4, 3)])
 def test_a_pinned_sweep_choice_is_run(system, choice, n):
     """While a choice is pinned the sweeps are launches of their own, with that choice: at least the
