@@ -347,6 +347,7 @@ struct PcgBatch {
 struct PcgResult {
     bool gave_up;  // at a barrier: p, rs, xs and the scalars hold no one iteration's state
     int iters;     // done; the last one judged the residual of the one before
+    bool undecided;  // they ended at the iteration limit
     double judged[MAX_BATCH], maxrr[MAX_BATCH];
     int flag[MAX_BATCH];
 };
@@ -386,6 +387,8 @@ size_t pcg_ctl_bytes();
 // launch without waiting; collect waits for the stream, and so for what was queued since
 int pcg_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B);
 int pcg_collect(c2q_ctx* ctx, const PcgBatch& B, PcgResult* out);
+// device memory, nonzero once the iterations have ended undecided
+const int* pcg_undecided(const PcgBatch& B);
 // Iterations of the FP64 CG on QplusQminus_eo in one cooperative launch
 // (pcg64.cu), with the context's solver scalars: until a judged residual is
 // below thr (from iteration min_iter on) or no number, or `iters` are done.

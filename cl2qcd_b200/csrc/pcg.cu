@@ -111,6 +111,8 @@ int pcg_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B)
     return pinned_copy(ctx, ctx->host_pinned_dev + PCG_PINNED, 0, prm.ctl, 0, sizeof(PcgCtl));
 }
 
+const int* pcg_undecided(const PcgBatch& B) { return &static_cast<const PcgCtl*>(B.ctl)->undecided; }
+
 int pcg_collect(c2q_ctx* ctx, const PcgBatch& B, PcgResult* out)
 {
     C2Q_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -121,7 +123,8 @@ int pcg_collect(c2q_ctx* ctx, const PcgBatch& B, PcgResult* out)
         ++ctx->barrier_giveups;
         return C2Q_OK;
     }
-    out->iters = c.iters;
+    out->iters     = c.iters;
+    out->undecided = c.undecided;
     for (int r = 0; r < B.n; ++r) {
         out->judged[r] = c.judged[r];
         out->maxrr[r]  = c.maxrr[r];

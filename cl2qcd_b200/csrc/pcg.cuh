@@ -35,7 +35,7 @@ struct PcgCtl {
     unsigned arrived;
     unsigned error;
     int iters;                  // iterations done
-    int pad_;
+    int undecided;              // they ended at the limit
     double judged[PK_MAX_RHS];  // the residual the last iteration judged
     double maxrr[PK_MAX_RHS];
     int flag[PK_MAX_RHS];       // SolverScalars::flag when it was judged
@@ -241,7 +241,10 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, 0>::MINB) pcg_kerne
             prm.ctl->maxrr[r]    = maxrr[r];
             prm.ctl->flag[r]     = judged_flag[r];
         }
-        if (threadIdx.x == 0) prm.ctl->iters = it;
+        if (threadIdx.x == 0) {
+            prm.ctl->iters     = it;
+            prm.ctl->undecided = !stop;
+        }
     }
 }
 

@@ -1,6 +1,7 @@
 // solvers.cu -- CG (FP64 and mixed precision with FP64 reliable updates),
 // BiCGStab (fast and save variants) and the eo Schur-complement inversion,
 // on top of the fused sweeps of fields.cu.
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstddef>
@@ -47,9 +48,19 @@ int make_fields(c2q_ctx* ctx, const c2q_lattice& lat, int prec, int n, Fields& F
     return C2Q_OK;
 }
 
+// Solves in progress on a device, all contexts together.
+std::atomic<int> solves_running[64];
+
 struct SolveClock {
     c2q_ctx* ctx;
-    explicit SolveClock(c2q_ctx* c) : ctx(c) { cudaEventRecord(ctx->ev0, ctx->stream); }
+    explicit SolveClock(c2q_ctx* c) : ctx(c)
+    {
+        solves_running[ctx->device & 63].fetch_add(1, std::memory_order_relaxed);
+        cudaEventRecord(ctx->ev0, ctx->stream);
+    }
+    ~SolveClock() { solves_running[ctx->device & 63].fetch_sub(1, std::memory_order_relaxed); }
+    SolveClock(const SolveClock&)            = delete;
+    SolveClock& operator=(const SolveClock&) = delete;
     double seconds()
     {
         cudaEventRecord(ctx->ev1, ctx->stream);
@@ -58,6 +69,19 @@ struct SolveClock {
         cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
         return ms * 1e-3;
     }
+};
+
+// Iterations of one cooperative launch at most.  Its blocks keep their places on the SMs
+// until it ends, so what other contexts queue waits for its end where it fills them (an
+// 8^4 request beside a 12^3x24 solve of 4 sources, p99 of its latency: 11.3 ms with launches up to
+// the next reliable update, 7.9 ms with these).  The results do not depend on it.
+bool alone(const c2q_ctx* ctx) { return solves_running[ctx->device & 63].load(std::memory_order_relaxed) <= 1; }
+int coop_iters(const c2q_ctx* ctx) { return alone(ctx) ? 100 : 16; }
+
+struct HaltScope {  // the context's launch predicate for a time
+    c2q_ctx* ctx;
+    HaltScope(c2q_ctx* c, const int* h) : ctx(c) { ctx->halt_dev = h; }
+    ~HaltScope() { ctx->halt_dev = nullptr; }
 };
 
 int read_sc(c2q_ctx* ctx, SolverScalars* h)
@@ -308,7 +332,7 @@ int cg_fp64(c2q_ctx* ctx, c2q_spinor_eo* x, int op, const c2q_gauge* g, const c2
                 S.p_ready = 1;
             }
             S.iter0       = iter;
-            S.iters       = std::min(end, (iter / P->iter_refresh + 1) * P->iter_refresh) - iter;
+            S.iters       = std::min(std::min(end, (iter / P->iter_refresh + 1) * P->iter_refresh) - iter, coop_iters(ctx));
             S.min_iter    = P->min_iter;
             S.lag         = lag;
             S.skip        = iter - 1 <= skip_upto;
@@ -810,18 +834,19 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
             C.delta  = delta;
             C.action = action;
             C.first  = iter == 0;
-            C.iters  = P->cgmax - iter;
+            C.iters  = std::min(P->cgmax - iter, coop_iters(ctx));
             C.ctl    = dsc + n;
             rc       = pcg_launch(ctx, g, gk, C);
-            // A right-hand side alone: whatever ended the iterations, its increment
+            // A right-hand side alone: if a decision ended the iterations, its increment
             // goes into x and the true residual is due, so both are queued behind them
-            // without asking.  The update that is expected to be the last takes the
+            // without asking (and skip their work where none did).  The update that is expected to be the last takes the
             // links as uploaded, as below: its residual has no room above thr.  (Where
             // the residual passed both levels in one step the guess is wrong, and the
             // true residual is computed again below.)
             const int k0 = act[0];
-            spec         = C.n == 1;
+            spec         = C.n == 1 && alone(ctx);
             if (!rc && spec) {
+                HaltScope undecided(ctx, pcg_undecided(C));
                 gk_spec = delta * delta * S[k0].maxrr * S[k0].maxrr < S[k0].thr ? G64 : gk64;
                 rc      = take_out(k0, nullptr);
                 if (!rc)
@@ -852,6 +877,7 @@ int cg_mixed_batch(c2q_ctx* ctx, c2q_spinor_eo* const* x, int op, const c2q_gaug
             for (int i = 0; i < C.n; ++i) {
                 RhsState& s = S[act[i]];
                 s.sweeps += per_apply * R.iters;
+                if (spec && R.undecided) s.sweeps -= per_apply;
                 s.maxrr        = R.maxrr[i];
                 judged[act[i]] = R.judged[i];
                 bad[act[i]]    = R.flag[i];
@@ -1299,12 +1325,6 @@ __global__ void bicg_end_kernel(SolverScalars* s, double* slot)
     flags[0]     = s->flag;
     flags[1]     = halt;
 }
-
-struct HaltScope {  // the context's launch predicate for the duration of a solve
-    c2q_ctx* ctx;
-    HaltScope(c2q_ctx* c, const int* h) : ctx(c) { ctx->halt_dev = h; }
-    ~HaltScope() { ctx->halt_dev = nullptr; }
-};
 
 // The device-driven iteration on an eo vector space: the field set, the
 // enqueueing of one fast or save iteration, and the residual ring.

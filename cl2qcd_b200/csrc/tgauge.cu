@@ -177,11 +177,13 @@ __global__ void __launch_bounds__(128) tg_to_inner_kernel(SpinorPtr<32> out, Spi
 }
 
 // x += G^dagger (xs + alpha p) on the parity-1 sites, xs = 0; one thread per slot
+// (halt: the context's launch predicate)
 template <int PB>
 __global__ void __launch_bounds__(128) tg_accumulate_kernel(SpinorPtr<64> x, SpinorPtr<32> xs, SpinorPtr<PB> p,
                                                             const SolverScalars* sc, const double2* __restrict__ G1,
-                                                            int n, int stride)
+                                                            int n, int stride, const int* halt)
 {
+    if (halt && *halt) return;
     const int j = blockIdx.x * blockDim.x + threadIdx.x, H = n / 2, ss = stride >> 1;
     if (j >= H) return;
     C2 b[12];
@@ -306,10 +308,10 @@ int tg_accumulate(c2q_ctx* ctx, const c2q_gauge* g, c2q_spinor_eo* x, c2q_spinor
     const unsigned blocks = (unsigned)((n / 2 + 127) / 128);
     if (p->prec == 16)
         tg_accumulate_kernel<16><<<blocks, 128, 0, ctx->stream>>>(sptr<64>(x), sptr<32>(xs), sptr<16>(p),
-                                                                          sc, G1, n, x->geom.stride);
+                                                                          sc, G1, n, x->geom.stride, ctx->halt_dev);
     else
         tg_accumulate_kernel<32><<<blocks, 128, 0, ctx->stream>>>(sptr<64>(x), sptr<32>(xs), sptr<32>(p),
-                                                                          sc, G1, n, x->geom.stride);
+                                                                          sc, G1, n, x->geom.stride, ctx->halt_dev);
     ctx->launches++;
     C2Q_CUDA(ctx, cudaGetLastError());
     return C2Q_OK;
