@@ -111,7 +111,7 @@ SIGNATURES = {
     "c2q_spinor_eo_convert": (C.c_int, [_P, _P]),
     "c2q_ctx_set_link_format": (C.c_int, [_P, C.c_int]),
     "c2q_ctx_trim": (C.c_int, [_P, C.POINTER(C.c_size_t)]),
-    "c2q_ctx_set_barrier_polls": (C.c_int, [_P, C.c_uint]),
+    "c2q_ctx_set_cooperative": (C.c_int, [_P, C.c_int]),
     "c2q_ctx_barrier_giveups": (C.c_longlong, [_P]),
     "c2q_ctx_set_autotune": (C.c_int, [_P, C.c_int]),
     "c2q_ctx_set_sweep_choice": (C.c_int, [_P, C.c_int]),

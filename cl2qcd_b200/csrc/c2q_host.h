@@ -90,9 +90,9 @@ struct c2q_ctx {
     // launch predicate of a device-driven solve (SolverScalars::halt): while set,
     // every reducing BLAS and dslash launch skips its work once *halt_dev != 0
     const int* halt_dev = nullptr;
-    // the cooperative CG iterations: polls of a wait at a grid barrier (0: none of these
-    // launches), and how many launches were given up
-    unsigned barrier_polls = 1u << 22;  // some seconds; a block of a resident grid arrives within microseconds
+    // the cooperative CG iterations (c2q_ctx_set_cooperative), and how many launches were
+    // given up at a barrier
+    int cooperative           = C2Q_COOPERATIVE_ON;
     long long barrier_giveups = 0;
     int sm_count  = 0;
     // pinned ring of the batched solvers: 4 slots x 16 right-hand sides x 4 doubles

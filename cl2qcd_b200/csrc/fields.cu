@@ -958,10 +958,12 @@ C2Q_EXPORT int c2q_ctx_create(c2q_ctx** out, int device, void* cuda_stream)
     return C2Q_OK;
 }
 
-C2Q_EXPORT int c2q_ctx_set_barrier_polls(c2q_ctx* ctx, unsigned polls)
+C2Q_EXPORT int c2q_ctx_set_cooperative(c2q_ctx* ctx, int mode)
 {
     if (!ctx) return C2Q_BAD_ARG;
-    ctx->barrier_polls = polls;
+    if (mode != C2Q_COOPERATIVE_OFF && mode != C2Q_COOPERATIVE_ON && mode != C2Q_COOPERATIVE_TEST)
+        return fail(ctx, C2Q_BAD_ARG, "unknown mode of the cooperative launches");
+    ctx->cooperative = mode;
     return C2Q_OK;
 }
 

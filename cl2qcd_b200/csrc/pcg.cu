@@ -40,7 +40,7 @@ int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* tiles, i
     *tiles = (g.seo / 2 + PK_THREADS - 1) / PK_THREADS;
     *room  = 0;
     // (per-launch timing and a pinned sweep choice want the sweeps as launches of their own)
-    if (ctx->profiling || ctx->force_choice >= 0 || !ctx->barrier_polls) return C2Q_OK;
+    if (ctx->profiling || ctx->force_choice >= 0 || !ctx->cooperative) return C2Q_OK;
     return prec == 16 ? (gkind_is_r12(gkind) ? pcg_resident<16, 6>(ctx, room) : pcg_resident<16, 9>(ctx, room))
                       : (gkind_is_r12(gkind) ? pcg_resident<32, 6>(ctx, room) : pcg_resident<32, 9>(ctx, room));
 }
@@ -57,6 +57,8 @@ static int pcg_go(c2q_ctx* ctx, PcgParams& prm)
     const void* kern      = (const void*)pcg_kernel<P, NL>;
     const int blocks      = prm.ntiles * prm.nrhs;  // pcg_capacity holds them all
     C2Q_CUDA(ctx, cudaMemsetAsync(prm.ctl, 0, sizeof(PcgCtl), ctx->stream));
+    if (ctx->cooperative == C2Q_COOPERATIVE_TEST)  // arrived: -1
+        C2Q_CUDA(ctx, cudaMemsetAsync(&prm.ctl->arrived, 0xFF, sizeof prm.ctl->arrived, ctx->stream));
     void* args[] = {&prm};
     C2Q_CUDA(ctx, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(PK_THREADS), args, smem, ctx->stream));
     ctx->launches++;
@@ -97,7 +99,6 @@ int pcg_launch(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const PcgBatch& B)
     prm.delta  = B.delta;
     prm.first  = B.first;
     prm.iters  = B.iters;
-    prm.polls  = ctx->barrier_polls;
     int rc     = ensure_partials(ctx, (size_t)prm.ntiles * PK_WARPS * B.n);
     if (rc) return rc;
     prm.partials = ctx->partials;

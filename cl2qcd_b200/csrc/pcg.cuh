@@ -57,7 +57,6 @@ struct PcgParams : PkStencil {
     int first;          // the solve's first iteration comes first: p is the residual, nothing to judge yet
     unsigned skip;      // bit r: the residual before the first iteration is a true one, not to be judged
     int iters;          // at most
-    unsigned polls;     // of a wait at a barrier
     double* partials;   // one per warp, tile and right-hand side
     PcgCtl* ctl;
 };
@@ -159,7 +158,7 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, 0>::MINB) pcg_kerne
                 else
                     SlotF32::store(F.p, ss, j, pv);
             }
-            if (!grid_barrier(&prm.ctl->arrived, &prm.ctl->error, target += gridDim.x, prm.polls, &ok)) return;
+            if (!grid_barrier(&prm.ctl->arrived, &prm.ctl->error, target += gridDim.x, &ok)) return;
         }
 #pragma unroll 1
         for (int ph = 0; ph < 4; ++ph) {
@@ -206,7 +205,7 @@ __global__ void __launch_bounds__(PK_THREADS, PkStage<P, NL, 0>::MINB) pcg_kerne
                 }
                 if (axpy) pk_partial<DOT_SELF>(dre, bc2(0.f), bc2(0.f), prm.partials, tile, nrhs, rhs);
             }
-            if (!grid_barrier(&prm.ctl->arrived, &prm.ctl->error, target += gridDim.x, prm.polls, &ok)) return;
+            if (!grid_barrier(&prm.ctl->arrived, &prm.ctl->error, target += gridDim.x, &ok)) return;
             if (axpy) {
                 pcg_sums(prm.partials, prm.ntiles * PK_WARPS, nrhs, tot, smem);
                 for (int r = threadIdx.x; r < nrhs; r += PK_THREADS) {

@@ -50,7 +50,6 @@ struct Params64 {
     int check_every;
     int iter0, min_iter;
     double thr;
-    unsigned polls;   // of a wait at a barrier
 };
 
 using C = Cplx<double>;
@@ -151,7 +150,7 @@ __global__ void __launch_bounds__(THREADS64, 2) pcg64_kernel(const Params64 prm)
                     const C v       = ldc(prm.r + at) - cmul(ldc(prm.p + at), mb);
                     prm.p[at]       = make_double2(v.re, v.im);
                 }
-            if (!grid_barrier(&prm.ctl->arrived, &prm.ctl->error, target += gridDim.x, prm.polls, &ok)) return;
+            if (!grid_barrier(&prm.ctl->arrived, &prm.ctl->error, target += gridDim.x, &ok)) return;
         }
 #pragma unroll 1
         for (int ph = 0; ph < 4; ++ph) {
@@ -254,7 +253,7 @@ __global__ void __launch_bounds__(THREADS64, 2) pcg64_kernel(const Params64 prm)
                     __syncthreads();  // the half spinors are read: the next tile may write its own
                 }
             }
-            if (!grid_barrier(&prm.ctl->arrived, &prm.ctl->error, target += gridDim.x, prm.polls, &ok)) return;
+            if (!grid_barrier(&prm.ctl->arrived, &prm.ctl->error, target += gridDim.x, &ok)) return;
             if (par) {
                 // one fixed order: thread j takes partials j, j + 256, ...
                 double s[1] = {0.0};
@@ -302,6 +301,8 @@ int blocks64(c2q_ctx* ctx, const void* kern, int ntiles, int* blocks)
 int go64(c2q_ctx* ctx, const void* kern, int blocks, Params64& prm)
 {
     C2Q_CUDA(ctx, cudaMemsetAsync(prm.ctl, 0, sizeof(Ctl64), ctx->stream));
+    if (ctx->cooperative == C2Q_COOPERATIVE_TEST)  // arrived: -1
+        C2Q_CUDA(ctx, cudaMemsetAsync(&prm.ctl->arrived, 0xFF, sizeof prm.ctl->arrived, ctx->stream));
     void* args[] = {&prm};
     C2Q_CUDA(ctx, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(THREADS64), args, 0, ctx->stream));
     ctx->launches++;
@@ -320,7 +321,7 @@ constexpr int PCG64_MAX_SITES = 24000;
 bool pcg64_applies(const c2q_ctx* ctx, int op, const c2q_gauge* gf)
 {
     // (per-launch timing wants the sweeps as launches of their own)
-    if (op != C2Q_OP_QPLUSQMINUS_EO || ctx->profiling || !ctx->barrier_polls || gf->geom.seo > PCG64_MAX_SITES)
+    if (op != C2Q_OP_QPLUSQMINUS_EO || ctx->profiling || !ctx->cooperative || gf->geom.seo > PCG64_MAX_SITES)
         return false;
     return adjoint_weights(gf);
 }
@@ -357,7 +358,6 @@ int pcg64_run(c2q_ctx* ctx, const c2q_gauge* g, int gkind, const Pcg64Solve& S, 
     prm.iter0       = S.iter0;
     prm.min_iter    = S.min_iter;
     prm.thr         = S.thr;
-    prm.polls       = ctx->barrier_polls;
     // the control block after the partials
     rc = ensure_partials(ctx, (size_t)prm.ntiles + 16);
     if (rc) return rc;

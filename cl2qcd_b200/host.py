@@ -102,9 +102,10 @@ class System:
         """Pin the launch choice of the reduced-precision sweeps (-1: the autotuner's)."""
         _check(self.lib.c2q_ctx_set_sweep_choice(self.h, choice), self.h, self.lib)
 
-    def set_barrier_polls(self, polls: int):
-        """Bound of a wait in the cooperative CG launches of small lattices (0: ordinary launches only)."""
-        _check(self.lib.c2q_ctx_set_barrier_polls(self.h, polls), self.h, self.lib)
+    def set_cooperative(self, mode: int):
+        """CG of small lattices: 0 ordinary launches only, 1 cooperative ones (default), 2 cooperative
+        ones whose barriers never complete (a test of the bound on their waits)."""
+        _check(self.lib.c2q_ctx_set_cooperative(self.h, mode), self.h, self.lib)
 
     @property
     def barrier_giveups(self) -> int:

@@ -306,10 +306,14 @@ C2Q_EXPORT int c2q_ctx_set_sweep_choice(c2q_ctx* ctx, int choice);
 C2Q_EXPORT int c2q_ctx_tune_report(const c2q_ctx* ctx, char* buf, int len);
 /* (no counterpart in the reference) On small lattices the CG on QplusQminus_eo runs many
  * iterations in one cooperative launch, whose blocks wait for each other at barriers.  A
- * wait ends after `polls` polls (default 2^22, some seconds); the launch is then given
- * up and the solve goes on with ordinary launches from its true residual.  0: ordinary
- * launches from the start.  barrier_giveups counts the launches given up so far. */
-C2Q_EXPORT int c2q_ctx_set_barrier_polls(c2q_ctx* ctx, unsigned polls);
+ * wait of a fraction of a second ends the launch, and the solve goes on with ordinary
+ * launches from its true residual; barrier_giveups counts the launches given up so far.
+ * Modes: ordinary launches only; cooperative ones (default); cooperative ones whose
+ * barriers wait for a block that does not exist, so that the wait runs out (a test). */
+#define C2Q_COOPERATIVE_OFF 0
+#define C2Q_COOPERATIVE_ON 1
+#define C2Q_COOPERATIVE_TEST 2
+C2Q_EXPORT int c2q_ctx_set_cooperative(c2q_ctx* ctx, int mode);
 C2Q_EXPORT long long c2q_ctx_barrier_giveups(const c2q_ctx* ctx);
 /* convert_to_eoprec / convert_from_eoprec (physics/lattices/spinorfield_eo.cpp:372-410):
  * `full` is a host spinor[V]; `even` gets the sites with x+y+z+t even (FP64 fields). */

@@ -119,6 +119,7 @@ def test_kept_blocks_serve_other_contexts():
     """A field and its staging buffer fit although another context keeps what is missing."""
     import cl2qcd_b200 as c2q
     a, b = c2q.System(0), c2q.System(0)
+    a.trim()  # nothing unused is left in the device's pool
     gfs = [c2q.Gaugefield(a, c2q.Lattice(24, 48)) for _ in range(3)]  # 382 MB each
     for gf in gfs:
         gf._destroy()

@@ -144,8 +144,8 @@ def test_fp64_iterations(port, system, O, ns, nt, rec12, action, mode):
 @pytest.mark.parametrize("precision,mode", [(64, "rel_tol"), (64, "prec"), (64, "graph"), (32, "one"), (16, "one"),
                                             (16, "batch"), (16, "graph")])
 def test_a_barrier_that_gives_up(port, O, precision, mode):
-    """Waits of one poll run out at once: the launch is given up and the solve goes on without it.
-    The context works as before afterwards."""
+    """Barriers that one block too many is awaited at: the wait runs out, the launch is
+    given up and the solve goes on without it.  The context works as before afterwards."""
     import cl2qcd_b200 as c2q
     system = c2q.System(0)
     port.set_lattice(8, 16, 1.0, 0.0)
@@ -160,7 +160,7 @@ def test_a_barrier_that_gives_up(port, O, precision, mode):
                              **kw)
     want, rep = _solve(c2q, system, L, gf, srcs, P, add)
     assert system.barrier_giveups == 0
-    system.set_barrier_polls(1)
+    system.set_cooperative(2)
     xs, reps = _solve(c2q, system, L, gf, srcs, P, add)
     assert system.barrier_giveups == 1
     for k, s in enumerate(srcs):
@@ -168,7 +168,7 @@ def test_a_barrier_that_gives_up(port, O, precision, mode):
         assert np.linalg.norm(r - s) / np.linalg.norm(s) <= 1.5e-10
         # one iteration lost and the search direction begun anew; with prec a check interval of 10
         assert reps[k]["iterations"] <= rep[k]["iterations"] + 10
-    system.set_barrier_polls(1 << 22)
+    system.set_cooperative(1)
     again, _ = _solve(c2q, system, L, gf, srcs, P, add)
     assert all(np.array_equal(a, w) for a, w in zip(again, want)) and system.barrier_giveups == 1
     system.close()
