@@ -49,7 +49,7 @@ struct c2q_ctx {
         void* p      = nullptr;
         size_t bytes = 0;
     };
-    LinkBlock link_cache[32];
+    LinkBlock link_cache[256];
     c2q_ctx* next_ctx = nullptr;  // the process's contexts (also under that mutex)
     // ring of pinned buffers between pageable host arrays and the device (hostcopy.cu)
     void* hc_ring        = nullptr;
