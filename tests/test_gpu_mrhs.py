@@ -50,8 +50,16 @@ def test_batch_matches_single_solves(port, system, O, precision):
         assert d <= 1e-12, (k, d)
 
 
+@pytest.fixture(params=[0, 1], ids=["launches", "cooperative"])
+def iterations(request, system):
+    """The iterations as launches of their own (which use_graph captures), or cooperative ones."""
+    system.set_cooperative(request.param)
+    yield request.param
+    system.set_cooperative(1)
+
+
 @pytest.mark.parametrize("precision", [32, 16])
-def test_twelve_point_sources_with_graphs(port, system, O, precision):
+def test_twelve_point_sources_with_graphs(port, system, O, precision, iterations):
     """12 spin-colour point sources at the origin, one batch, graph-captured iterations."""
     import cl2qcd_b200 as c2q
     L, g, gf = _problem(port, c2q, system, 8, 8, 0.25, 7)
@@ -73,7 +81,7 @@ def test_twelve_point_sources_with_graphs(port, system, O, precision):
         assert np.linalg.norm(r - srcs[k]) <= 1.5e-10
 
 
-def test_more_sources_than_one_batch(port, system, O):
+def test_more_sources_than_one_batch(port, system, O, iterations):
     """17 sources: one batch of 16 and one of 1, FP16, graph-captured."""
     import cl2qcd_b200 as c2q
     L, g, gf = _problem(port, c2q, system, 4, 8, 0.3, 11)

@@ -114,11 +114,15 @@ def test_cg_true_residual_1e10(port, system, O, precision, rec12):
     assert np.linalg.norm(r - b) / np.linalg.norm(b) <= 1.5e-10
 
 
+@pytest.mark.parametrize("cooperative", [0, 1])
 @pytest.mark.parametrize("iter_refresh", [100, 7])
-def test_fp64_cg_graph_replay_matches_eager(port, system, O, iter_refresh):
+def test_fp64_cg_graph_replay_matches_eager(port, system, O, iter_refresh, cooperative, request):
     """FP64 CG with use_graph: the iterations between refreshes replay as a
     captured graph of the same kernels, so the iterates are bitwise those of the
-    eager loop (also across refreshes, iter_refresh 7)."""
+    eager loop (also across refreshes, iter_refresh 7).  Cooperative launches, the default on
+    this lattice, ignore use_graph."""
+    system.set_cooperative(cooperative)
+    request.addfinalizer(lambda: system.set_cooperative(1))
     import cl2qcd_b200 as c2q
     L, g, gf, b = _prob(port, c2q, system, 8, 8, 0.3, 1)
     add = c2q.AdditionalParameters(0.15, 2 * 0.15 * 0.01)

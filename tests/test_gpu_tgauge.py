@@ -71,8 +71,16 @@ def test_solve_in_temporal_gauge(port, system, O, precision, case):
     assert d <= 1e-8, d
 
 
+@pytest.fixture(params=[0, 1], ids=["launches", "cooperative"])
+def iterations(request, system):
+    """The iterations as launches of their own (which use_graph captures), or cooperative ones."""
+    system.set_cooperative(request.param)
+    yield request.param
+    system.set_cooperative(1)
+
+
 @pytest.mark.parametrize("precision", [32, 16])
-def test_batch_in_temporal_gauge_matches_single(port, system, O, precision):
+def test_batch_in_temporal_gauge_matches_single(port, system, O, precision, iterations):
     """A batch of four sources in the temporal gauge (graph-captured) gives each
     source the result it gets alone."""
     import cl2qcd_b200 as c2q
