@@ -1,5 +1,6 @@
 // blas.cuh -- eo spinor-field level-1 BLAS, fused CG updates, reductions and
-// layout conversions, one thread per eo site, any storage precision.
+// layout conversions of FP64 fields, one thread per eo site (FP32 / FP16 fields:
+// blas_pk.cuh, which shares the arguments declared here).
 //
 // Semantics follow the reference's eo BLAS (physics/lattices/spinorfield_eo.cpp
 // and ocl_kernel/spinorfield_eo_*.cl), including its sign convention
@@ -60,6 +61,7 @@ struct BlasArgs {
 template <int P>
 __global__ void __launch_bounds__(BLAS_THREADS) blas_kernel(const BlasArgs<P> A)
 {
+    static_assert(P == 64, "FP32 / FP16 fields take blas_pk_kernel");
     pdl_enter();
     if (halted(A.red)) return;  // a stopped device-driven solve: every block leaves
     using R      = typename Prec<P>::R;
@@ -229,18 +231,15 @@ __global__ void __launch_bounds__(BLAS_THREADS) cg_p_kernel(const CgPArgs<P> A)
     SpinorIO<P>::store(A.p, A.stride, i, p);
 }
 
-// Precision conversion of a whole eo field (same site order and stride).
-template <int PO, int PI>
-__global__ void __launch_bounds__(BLAS_THREADS) convert_kernel(SpinorPtr<PO> out, SpinorPtr<PI> in, int n, int stride)
+// An FP64 field into another (the conversions with FP32 / FP16 fields: blas_pk.cuh).
+static __global__ void __launch_bounds__(BLAS_THREADS) convert64_kernel(SpinorPtr<64> out, SpinorPtr<64> in, int n,
+                                                                        int stride)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    Cplx<typename Prec<PI>::R> a[12];
-    Cplx<typename Prec<PO>::R> b[12];
-    SpinorIO<PI>::load(in, stride, i, a);
-#pragma unroll
-    for (int k = 0; k < 12; ++k) b[k] = {(typename Prec<PO>::R)a[k].re, (typename Prec<PO>::R)a[k].im};
-    SpinorIO<PO>::store(out, stride, i, b);
+    Cplx<double> a[12];
+    SpinorIO<64>::load(in, stride, i, a);
+    SpinorIO<64>::store(out, stride, i, a);
 }
 
 // ---- layout conversion between the reference's AoS host formats and SoA ----

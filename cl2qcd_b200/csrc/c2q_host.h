@@ -355,9 +355,11 @@ struct PcgResult {
 // of the device, 0 where these iterations are not to be taken.  A batch takes them if
 // every tile of every right-hand side has a resident block of its own (one
 // wave).  With more, a phase runs a second, partly empty wave between two
-// barriers and the ordinary launches are as fast or faster: FP16, per iteration
-// with its share of the reliable updates, 16^3x32 (256 tiles) 53 us against 69 us,
-// 20^3x40 (625 tiles) 110 against 104, four sources at 16^3x32 165 against 144.
+// barriers and the ordinary launches are as fast or faster: FP16, a solve's time over its
+// iterations, against the ordinary launches replayed as a graph, 16^3x32 (256 tiles, one
+// wave of 444 blocks) 39 us against 48 us, 12^3x24 with five sources (405) 64.5 against
+// 65.0; 16^3x32 with two sources (512) 89 against 71, 20^3x40 (625) 90 against 80, four sources
+// at 16^3x32 133 against 111.
 int pcg_capacity(c2q_ctx* ctx, int prec, int gkind, const Geom& g, int* tiles, int* room);
 // Blocks of cooperative CG launches in flight on a device, all contexts together.  The
 // hardware starts such a launch only once all its blocks have room, so grids that do

@@ -785,7 +785,7 @@ static void convert_go(c2q_ctx* ctx, c2q_spinor_eo* out, const c2q_spinor_eo* in
 {
     const int n = out->geom.seo;
     if constexpr (PO == 64 && PI == 64)
-        convert_kernel<PO, PI><<<(n + BLAS_THREADS - 1) / BLAS_THREADS, BLAS_THREADS, 0, ctx->stream>>>(
+        convert64_kernel<<<(n + BLAS_THREADS - 1) / BLAS_THREADS, BLAS_THREADS, 0, ctx->stream>>>(
             sptr<PO>(out), sptr<PI>(in), n, out->geom.stride);
     else
         convert_pk_kernel<PO, PI><<<(n / 2 + BLAS_PK_THREADS - 1) / BLAS_PK_THREADS, BLAS_PK_THREADS, 0, ctx->stream>>>(

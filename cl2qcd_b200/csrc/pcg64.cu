@@ -312,10 +312,10 @@ int go64(c2q_ctx* ctx, const void* kern, int blocks, Params64& prm)
 }  // namespace
 
 // Lattices of at most this many eo sites take the cooperative iterations: a
-// phase is then at most about two and a half waves of tiles.  Per iteration, against
-// the ordinary launches replayed as a graph: 8^4 21.5 us against 52.6, 12^3x16 (13824
-// sites) 37.9 against 53.8, 12^3x24 (20736) 51.6 against 56.4, 16^4 (32768) 62.7
-// against 60.5.
+// phase is then at most about two and a half waves of tiles.  A solve's time over its
+// iterations (its fixed part included), against the ordinary launches replayed as a
+// graph: 8^4 19.3 us against 46.4, 12^3x16 (13824 sites) 37.3 against 45.8, 12^3x24
+// (20736) 51.2 against 50.0, 16^4 (32768) 60.8 against 52.6.
 constexpr int PCG64_MAX_SITES = 24000;
 
 bool pcg64_applies(const c2q_ctx* ctx, int op, const c2q_gauge* gf)

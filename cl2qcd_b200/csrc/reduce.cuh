@@ -1,14 +1,16 @@
 // reduce.cuh -- deterministic global reductions fused into the producing kernel.
 //
-// Every reducing kernel writes one partial per block into a scratch array, in
-// block order.  The last block to finish (an atomic ticket, reset by that
-// block) sums the partials in a fixed order with a fixed tree, so the result
-// is independent of block scheduling and bitwise reproducible for a given
+// The FP64 sweeps, the BLAS and mix_update write one partial per block into a
+// scratch array, in block order, and the last block to finish (an atomic ticket, reset
+// by that block) sums them.  The paired-site sweeps (pdslash.cuh) write one per warp,
+// and a kernel behind them sums up; the cooperative iterations (pcg.cuh, pcg64.cu) sum
+// up in every block after a grid barrier.  Always in a fixed order with a fixed tree,
+// so the result is independent of block scheduling and bitwise reproducible for a given
 // launch shape.  No floating-point atomics are used anywhere.
 //
-// The same last block then runs a small scalar "finisher" on the device
-// (complex divisions for CG/BiCGStab coefficients), so solver iterations need
-// no host round trip.
+// Whoever has the sum then runs a small scalar "finisher" on the device (complex
+// divisions for CG/BiCGStab coefficients), so solver iterations need no host round
+// trip.
 #pragma once
 
 #include "c2q_internal.cuh"
@@ -69,7 +71,7 @@ enum HaltBits : int {
     HALT_CONV_NEXT = 16,
 };
 
-// What the last block does with the reduced value(s).
+// What is done with the reduced value(s).
 enum Finisher : int {
     FIN_STORE_RESULT = 0,  // result[0..NV) = sum
     FIN_CG_ALPHA     = 1,  // rho = sum; alpha = omega / rho
@@ -90,7 +92,7 @@ enum Finisher : int {
 
 struct RedArgs {
     double* partials;      // >= gridDim.x * NV doubles of scratch
-    unsigned* ticket;      // zero-initialised counter, reset by the last block
+    unsigned* ticket;      // zero-initialised counters, one per group, reset by its last block
     double* result;        // FIN_STORE_RESULT destination (NV doubles)
     SolverScalars* sc;     // solver scalars for the CG finishers
     int fin;
@@ -153,16 +155,7 @@ __device__ __forceinline__ void cdiv_store(double* out, const double* n, const d
     out[1] = (n[1] * d[0] - n[0] * d[1]) / norm;
 }
 
-// Partial `index` of a reduction (thread 0 holds the block sum).
-template <int NV>
-__device__ __forceinline__ void store_partial(const double v[NV], const RedArgs& ra, size_t index)
-{
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) ra.partials[index * NV + k] = v[k];
-}
-
-// What the last block's thread 0 does with the group's sum (RedArgs::fin).
+// What one thread does with the group's sum (RedArgs::fin).
 template <int NV>
 __device__ __forceinline__ void finish_apply(const RedArgs& ra, const double acc[NV])
 {
@@ -271,30 +264,25 @@ __device__ __forceinline__ void finish_apply(const RedArgs& ra, const double acc
 // and its last block sums that group's partials in block order.
 template <int NV>
 __device__ __forceinline__ void finish_reduction(const double v[NV], const RedArgs& ra, double* smem, int grp = 0,
-                                                 int G = 1);
-
-// The ticket and final sum of a group whose `nparts` partials sit at
-// partials[(m * G + grp) * NV], m < nparts, written by the `nblocks` blocks of
-// the group (grid-stride kernels write several partials per block).
-// ROUND: partials loaded per thread before they are added (the order of the
-// additions does not depend on it); wider rounds shorten this block's serial
-// tail, at ROUND * NV registers.
-template <int NV, int ROUND = 8>
-__device__ __forceinline__ void finish_group(const RedArgs& ra, double* smem, int grp, int G, int nparts, int nblocks)
+                                                 int G = 1)
 {
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) ra.partials[(size_t)blockIdx.x * NV + k] = v[k];
+    const int nb = (int)gridDim.x / G;  // blocks (= partials) of this group
     __shared__ bool last;
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned t = atomicAdd(ra.ticket + grp, 1u);
-        last             = (t == (unsigned)nblocks - 1u);
+        last             = (t == (unsigned)nb - 1u);
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    const int nb = nparts;
     // fixed-order sum of the group's partials: thread j takes partials
-    // j, j + blockDim.x, ... in rounds of ROUND independent loads (this block
+    // j, j + blockDim.x, ... in rounds of independent loads (this block
     // runs alone at the end of the kernel, so its load latency is not hidden)
+    constexpr int ROUND = 8;
     double acc[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] = 0.0;
@@ -318,14 +306,6 @@ __device__ __forceinline__ void finish_group(const RedArgs& ra, double* smem, in
         finish_apply<NV>(ra, acc);
         __threadfence();
     }
-}
-
-template <int NV>
-__device__ __forceinline__ void finish_reduction(const double v[NV], const RedArgs& ra, double* smem, int grp, int G)
-{
-    store_partial<NV>(v, ra, blockIdx.x);
-    const int nb = (int)gridDim.x / G;  // blocks (= partials) of this group
-    finish_group<NV>(ra, smem, grp, G, nb, nb);
 }
 
 }  // namespace c2q

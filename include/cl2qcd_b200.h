@@ -221,7 +221,9 @@ C2Q_EXPORT long long c2q_ctx_launch_count(const c2q_ctx* ctx);
  * precision `prec` (64, 32, 16), the number of timed launches, their summed
  * device time in milliseconds and their summed algorithmic bytes (per output
  * site: 8 links, the input and output spinors, and the spinors an epilogue or
- * a fused reduction reads at the output site). */
+ * a fused reduction reads at the output site).  While it is on, the CGs of small lattices
+ * run each sweep as a launch of its own (else: c2q_ctx_set_cooperative) and use_graph has
+ * no effect, so a solve's time then is not that of the same solve without it. */
 C2Q_EXPORT int c2q_ctx_profile(c2q_ctx* ctx, int enable);
 C2Q_EXPORT int c2q_ctx_profile_read(c2q_ctx* ctx, int prec, long long* launches, double* total_ms,
                                     double* bytes);
